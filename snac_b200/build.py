@@ -44,7 +44,7 @@ def stale() -> bool:
 def build(force: bool = False, verbose: bool = False, defines=(), out: str = LIB) -> str:
     if not force and not stale() and out == LIB:
         return LIB
-    cmd = [nvcc(), *ARCH, *["-D" + d for d in defines], "-lineinfo", "-O3", "-fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
+    cmd = [nvcc(), *ARCH, *["-D" + d for d in defines], "-lineinfo", "-O3", "-split-compile=0", "-fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
            "-shared", "-I" + os.path.join(ROOT, "include"), "-o", out + ".tmp",
            os.path.join(CSRC, "snac_api.cu")]
     if verbose:

@@ -239,9 +239,9 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     double s_mid[6];  // stress after each in-place rotation update (for the reverse)
     double r01 = 0, r02 = 0, r12 = 0;
     if (rotate) {
-        rotate_stress(v, g, dt, s_pre);
         double r[3];
-        spin_rates(v, g, r);  // the same values rotate_stress used
+        spin_rates(v, g, r, false);
+        rotate_stress(r, dt, s_pre);
         r01 = r[0];
         r02 = r[1];
         r12 = r[2];
@@ -250,7 +250,7 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     for (int a = 0; a < 6; a++) s_mid[a] = s_pre[a];
 
     double sr[6];
-    tet_strain_rate(v, g, sr);
+    tet_strain_rate(v, g, sr, false);
     double sr_raw[6];
 #pragma unroll
     for (int a = 0; a < 6; a++) sr_raw[a] = sr[a];

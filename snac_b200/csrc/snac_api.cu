@@ -75,6 +75,7 @@ struct snac_gpu {
     int has_density = 0;
     int n_phases = 0;
     double wave_speed = 0.0;
+    int n_sm = 148;
     cudaStream_t stream = nullptr;
     bool own_stream = true;  // false for the models of a batch, which share the batch's stream
     long long alloc_bytes = 0;  // device bytes allocated for this handle since creation (snac_gpu_device_bytes)
@@ -93,8 +94,6 @@ struct snac_gpu {
     double* hflux = nullptr;
     double* tpre = nullptr;
     double* fterm = nullptr;
-    double* fgrav = nullptr;
-    double* fmass = nullptr;
     uchar4* bc = nullptr;
     double* vbc_val = nullptr;
     double* tbc_val = nullptr;
@@ -244,8 +243,6 @@ Fields fields_at(const snac_gpu* h, int parity) {
     F.hflux = h->hflux;
     F.tpre = h->tpre;
     F.fterm = h->fterm;
-    F.fgrav = h->fgrav;
-    F.fmass = h->fmass;
     F.bc = h->bc;
     F.vbc_val = h->vbc_val;
     F.tbc_val = h->tbc_val;
@@ -263,7 +260,33 @@ Fields fields_at(const snac_gpu* h, int parity) {
 Fields fields(const snac_gpu* h) { return fields_at(h, h->parity); }
 
 unsigned elem_blocks(const Mesh& m) { return (unsigned)((m.ne + ELEM_PER_BLOCK - 1) / ELEM_PER_BLOCK); }
-unsigned node_blocks(const Mesh& m) { return (unsigned)((m.nn + 127) / 128); }
+
+// The launch of a node gather over blocks of NODE_THREADS nodes; rows: of a
+// stage.  As many stages as the grid leaves shared memory for: four (107 KB
+// of a momentum gather) up to two blocks per SM, two up to four, else one.
+struct NodeLaunch {
+    unsigned blocks;
+    int stages;
+    size_t smem;
+};
+NodeLaunch node_launch(const snac_gpu* h, unsigned blocks, int rows) {
+    NodeLaunch l;
+    l.blocks = blocks;
+    const unsigned sms = (unsigned)h->n_sm;
+    l.stages = blocks <= 2 * sms ? 4 : blocks <= 4 * sms ? 2 : 1;
+    l.smem = (size_t)l.stages * gather_stage_bytes(rows, NODE_THREADS);
+    return l;
+}
+unsigned node_blocks(const Mesh& m) { return (unsigned)((m.nn + NODE_THREADS - 1) / NODE_THREADS); }
+int force_rows(const snac_gpu* h) {
+    const bool cdt = h->cfg.dt_type == SNAC_DT_CONSTANT;
+    return force_chunk(cdt) + force_tail(cdt, h->cfg.vonly != 0);
+}
+template <class K>
+cudaError_t allow_smem(K kernel, size_t bytes) {
+    return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+                             : cudaSuccess;
+}
 
 // called right after each launch: checks it and, when profiling, records an
 // event behind it (the event before the first launch is recorded by the caller)
@@ -346,7 +369,9 @@ int op_fused_stress(snac_gpu* h) {
 
 int op_energy_nodes(snac_gpu* h, int count_step = 0) {
     if (!h->temperature) return 0;
-    k_heat_nodes<<<node_blocks(h->mesh), 128, 0, h->stream>>>(h->mesh, fields(h), h->cfg, count_step);
+    const NodeLaunch l = node_launch(h, node_blocks(h->mesh), HEAT_CHUNK + HEAT_TAIL);
+    CK(allow_smem(k_heat_nodes, l.smem));
+    k_heat_nodes<<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, fields(h), h->cfg, count_step, l.stages);
     h->launches++;
     if (count_step) h->time_step++;
     return launch_check_named(h, "k_heat_nodes");
@@ -369,26 +394,28 @@ int op_calc_stresses(snac_gpu* h) {
     return launch_check_named(h, "k_calc_stresses");
 }
 
+template <int DT, bool VO>
+int launch_loop_nodes(snac_gpu* h, const Fields& F) {
+    const NodeLaunch l = node_launch(h, node_blocks(h->mesh), force_rows(h));
+    CK(allow_smem(k_loop_nodes<DT, VO>, l.smem));
+    k_loop_nodes<DT, VO><<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, F, h->cfg, l.stages);
+    return 0;
+}
 int op_loop_nodes(snac_gpu* h) {
     Fields F = fields(h);
-    const unsigned nb = node_blocks(h->mesh);
     const bool vo = h->cfg.vonly != 0;
+    int rc;
     switch (h->cfg.dt_type) {
-        case SNAC_DT_CONSTANT:
-            k_loop_nodes<SNAC_DT_CONSTANT, false><<<nb, 128, 0, h->stream>>>(h->mesh, F, h->cfg);
-            break;
+        case SNAC_DT_CONSTANT: rc = launch_loop_nodes<SNAC_DT_CONSTANT, false>(h, F); break;
         case SNAC_DT_DYNAMIC:
-            if (vo) k_loop_nodes<SNAC_DT_DYNAMIC, true><<<nb, 128, 0, h->stream>>>(h->mesh, F, h->cfg);
-            else k_loop_nodes<SNAC_DT_DYNAMIC, false><<<nb, 128, 0, h->stream>>>(h->mesh, F, h->cfg);
+            rc = vo ? launch_loop_nodes<SNAC_DT_DYNAMIC, true>(h, F) : launch_loop_nodes<SNAC_DT_DYNAMIC, false>(h, F);
             break;
-        default:
-            if (vo) k_loop_nodes<SNAC_DT_WAVE, true><<<nb, 128, 0, h->stream>>>(h->mesh, F, h->cfg);
-            else k_loop_nodes<SNAC_DT_WAVE, false><<<nb, 128, 0, h->stream>>>(h->mesh, F, h->cfg);
-            break;
+        default: rc = vo ? launch_loop_nodes<SNAC_DT_WAVE, true>(h, F) : launch_loop_nodes<SNAC_DT_WAVE, false>(h, F);
     }
+    if (rc) return rc;
     h->launches++;
     h->parity ^= 1;  // the new coordinates are current from here on
-    int rc = launch_check_named(h, "k_loop_nodes");
+    rc = launch_check_named(h, "k_loop_nodes");
     if (rc || !topo_on(h->cfg)) return rc;
     k_topo<<<1, 1024, 0, h->stream>>>(h->mesh, h->pos[h->parity ^ 1], h->pos[h->parity], h->cfg, h->sc, h->topo_scratch);
     h->launches++;
@@ -633,24 +660,28 @@ int op_calc_stresses_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     return launch_check_named(h, "k_calc_stresses_slab");
 }
 
+template <int DT, bool VO>
+int launch_loop_nodes_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
+    const NodeLaunch l = node_launch(h, (unsigned)(b1 - b0), force_rows(h));
+    CK(allow_smem(k_loop_nodes_slab<DT, VO>, l.smem));
+    k_loop_nodes_slab<DT, VO><<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, F, h->cfg, b0, l.stages);
+    return 0;
+}
 int op_loop_nodes_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     if (b1 <= b0) return 0;
-    const unsigned nb = (unsigned)(b1 - b0);
     const bool vo = h->cfg.vonly != 0;
-    cudaStream_t st = h->stream;
+    int rc;
     switch (h->cfg.dt_type) {
-        case SNAC_DT_CONSTANT:
-            k_loop_nodes_slab<SNAC_DT_CONSTANT, false><<<nb, 128, 0, st>>>(h->mesh, F, h->cfg, b0);
-            break;
+        case SNAC_DT_CONSTANT: rc = launch_loop_nodes_slab<SNAC_DT_CONSTANT, false>(h, F, b0, b1); break;
         case SNAC_DT_DYNAMIC:
-            if (vo) k_loop_nodes_slab<SNAC_DT_DYNAMIC, true><<<nb, 128, 0, st>>>(h->mesh, F, h->cfg, b0);
-            else k_loop_nodes_slab<SNAC_DT_DYNAMIC, false><<<nb, 128, 0, st>>>(h->mesh, F, h->cfg, b0);
+            rc = vo ? launch_loop_nodes_slab<SNAC_DT_DYNAMIC, true>(h, F, b0, b1)
+                    : launch_loop_nodes_slab<SNAC_DT_DYNAMIC, false>(h, F, b0, b1);
             break;
         default:
-            if (vo) k_loop_nodes_slab<SNAC_DT_WAVE, true><<<nb, 128, 0, st>>>(h->mesh, F, h->cfg, b0);
-            else k_loop_nodes_slab<SNAC_DT_WAVE, false><<<nb, 128, 0, st>>>(h->mesh, F, h->cfg, b0);
-            break;
+            rc = vo ? launch_loop_nodes_slab<SNAC_DT_WAVE, true>(h, F, b0, b1)
+                    : launch_loop_nodes_slab<SNAC_DT_WAVE, false>(h, F, b0, b1);
     }
+    if (rc) return rc;
     h->launches++;
     return launch_check_named(h, "k_loop_nodes_slab");
 }
@@ -681,7 +712,9 @@ int op_heat_flux_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
 
 int op_heat_nodes_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     if (b1 <= b0) return 0;
-    k_heat_nodes_slab<<<(unsigned)(b1 - b0), 128, 0, h->stream>>>(h->mesh, F, h->cfg, b0);
+    const NodeLaunch l = node_launch(h, (unsigned)(b1 - b0), HEAT_CHUNK + HEAT_TAIL);
+    CK(allow_smem(k_heat_nodes_slab, l.smem));
+    k_heat_nodes_slab<<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, F, h->cfg, b0, l.stages);
     h->launches++;
     return launch_check_named(h, "k_heat_nodes_slab");
 }
@@ -895,7 +928,7 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
     {
         int dev = 0, sms = 0;
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-            c.prefetch_ahead = sms * SNAC_ELEM_MINB;
+            h->n_sm = sms;
     }
     c.pisos = d->pisos;  // replaced below when the hydrostatic IC runs here
     c.rzbo = d->rzbo;
@@ -907,12 +940,18 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
     }
 
     const long long ne = m.ne, nn = m.nn, nq = ne * NT;
+    const long long ngroups = (ne + GROUP - 1) / GROUP;
+    // the volume alone stands for the gravity and inertial-mass terms (Config::vonly)
+    c.vonly = !d->element_material && !h->has_density && d->dt_type != SNAC_DT_CONSTANT;
+    {
+        const bool cdt = d->dt_type == SNAC_DT_CONSTANT;
+        m.frows = 4 * force_chunk(cdt) + force_tail(cdt, c.vonly != 0);
+    }
     int rc = 0;
     if ((rc = dalloc(h, &h->pos[0], nn)) || (rc = dalloc(h, &h->pos[1], nn)) || (rc = dalloc(h, &h->vel, nn)) ||
         (rc = dalloc(h, &h->force, nn)) || (rc = dalloc(h, &h->stress, nq * 6)) || (rc = dalloc(h, &h->bc, nn)) ||
         (rc = dalloc(h, &h->sc, 1)) || (rc = dalloc(h, &h->mats, MAX_PHASES)) ||
-        (rc = dalloc(h, &h->fterm, m.ner * NT * 12)) || (rc = dalloc(h, &h->fgrav, m.ner * NT)) ||
-        (rc = dalloc(h, &h->fmass, m.ner * NT * (d->dt_type == SNAC_DT_CONSTANT ? 4 : 1))))
+        (rc = dalloc(h, &h->fterm, ngroups * m.frows * GROUP)))
         return rc;
     if (d->constitutive == SNAC_RHEOLOGY_PLASTIC || d->constitutive == SNAC_RHEOLOGY_VISCOPLASTIC)
         if ((rc = dalloc(h, &h->eps_p, nq))) return rc;
@@ -928,7 +967,7 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
     if (topo_on(c))
         if ((rc = dalloc(h, &h->topo_scratch, (size_t)m.nnx * m.nnz))) return rc;
     if (d->temperature) {
-        if ((rc = dalloc(h, &h->hflux, m.ner * NT * HF_STRIDE))) return rc;
+        if ((rc = dalloc(h, &h->hflux, ngroups * HROWS * GROUP))) return rc;
         if (h->has_density && (rc = dalloc(h, &h->tpre, nn))) return rc;
     }
 
@@ -1034,8 +1073,6 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
     for (int p = 0; p < d->n_materials; p++)  // Drucker-Prager controls: Context.c:851-854 defaults 1 and 1e-3
         dm[p] = to_dev(d->materials[p], d->element_friction_scale != nullptr,
                        d->dp_max_iterations ? d->dp_max_iterations[p] : 1, d->dp_tolerance ? d->dp_tolerance[p] : 1.e-3);
-    // the volume alone stands for the gravity and inertial-mass terms (Config::vonly)
-    h->cfg.vonly = SNAC_VOLUME_ONLY && !d->element_material && !h->has_density && d->dt_type != SNAC_DT_CONSTANT;
     if (d->element_material) {
         std::vector<unsigned char> mt(ne);
         for (long long e = 0; e < ne; e++) {
@@ -1130,7 +1167,7 @@ void snac_gpu_destroy(snac_gpu* h) {
         delete q;
     }
     void* bufs[] = {h->pos[0], h->pos[1], h->vel, h->force, h->stress, h->eps_p, h->pst, h->visc, h->density, h->vol,
-                    h->hflux, h->tpre, h->fterm, h->fgrav, h->fmass, h->bc, h->vbc_val, h->tbc_val, h->mat, h->mats, h->coh_scale, h->fric_scale,
+                    h->hflux, h->tpre, h->fterm, h->bc, h->vbc_val, h->tbc_val, h->mat, h->mats, h->coh_scale, h->fric_scale,
                     h->visc_scale, h->sc, h->stage, h->escal, h->residual_fr, h->topo_scratch};
     for (void* b : bufs)
         if (b) cudaFree(b);
@@ -1433,7 +1470,7 @@ static int record_host_step(snac_gpu* h, const snac_state_view* in, const snac_s
         const int s = o.stage, i = o.slab;
         if (s == 0) CK(cudaStreamWaitEvent(h->stream, q->ev_in[i], 0));
         const int b0 = (int)(E[i] / ELEM_PER_BLOCK), b1 = (int)((E[i + 1] + ELEM_PER_BLOCK - 1) / ELEM_PER_BLOCK);
-        const int n0 = (int)(N[i] / 128), n1 = (int)((N[i + 1] + 127) / 128);
+        const int n0 = (int)(N[i] / NODE_THREADS), n1 = (int)((N[i + 1] + NODE_THREADS - 1) / NODE_THREADS);
         switch (stages[s]) {
             case HEAT_FLUX: rc = op_heat_flux_slab(h, F0, b0, b1); break;
             case HEAT_NODES: rc = op_heat_nodes_slab(h, F0, n0, n1); break;
@@ -1745,7 +1782,9 @@ int blaunch_elem(snac_gpu_batch* b, const ModelDesc* D, const snac_gpu_batch::Li
 template <int OP>
 int blaunch_nodes(snac_gpu_batch* b, const ModelDesc* D, const snac_gpu_batch::List& L, int threads) {
     if (L.n == 0) return 0;
-    kb_nodes<OP><<<tile_grid(b, L.n, b->tune.node_blocks_per_sm), threads, 0, b->stream>>>(D, b->tiles + L.off, L.n);
+    const size_t smem = OP == BOP_MINLS ? 0 : node_stage_bytes(OP, threads);
+    BCK(allow_smem(kb_nodes<OP>, smem));
+    kb_nodes<OP><<<tile_grid(b, L.n, b->tune.node_blocks_per_sm), threads, smem, b->stream>>>(D, b->tiles + L.off, L.n);
     return bcheck_launch(b, "kb_nodes");
 }
 

@@ -54,82 +54,66 @@ __device__ __forceinline__ void load_desc(ModelDesc& dst, const ModelDesc* __res
 
 // the element bodies for a tile's model: phase 0 from the descriptor (in
 // shared memory) when the model has one phase, else the model's phase table
-template <int P>
-__device__ __forceinline__ void fused_step_any(const ModelDesc& md, int lb, bool count_step = true) {
+union TileSmem {
+    ElemSmem elem;
+    HeatSmem heat;
+};
+template <int P, bool FUSED>
+__device__ __forceinline__ void stress_any(TileSmem& S, const ModelDesc& md, int lb) {
     if (md.F.mat)
-        k_fused_step_body<P, false>(md.m, md.F, md.cfg, lb, count_step);
+        stress_group<P, false, FUSED>(S.elem, md.m, md.F, md.cfg, lb);
     else
-        k_fused_step_body<P, true>(md.m, md.F, md.cfg, lb, count_step);
+        stress_group<P, true, FUSED>(S.elem, md.m, md.F, md.cfg, lb);
 }
-template <int P>
-__device__ __forceinline__ void calc_stresses_any(const ModelDesc& md, int lb) {
+__device__ __forceinline__ void heat_flux_any(TileSmem& S, const ModelDesc& md, int lb) {
     if (md.F.mat)
-        k_calc_stresses_body<P, false>(md.m, md.F, md.cfg, lb);
+        heat_group<false, false>(S.heat, md.m, md.F, md.cfg, lb);
     else
-        k_calc_stresses_body<P, true>(md.m, md.F, md.cfg, lb);
+        heat_group<true, false>(S.heat, md.m, md.F, md.cfg, lb);
+}
+// a model's first launch of a fused step: timeStep++, currentTime += dt
+// (once per model), then the pending element update with the stress update,
+// or with temperature the heat flux
+__device__ __forceinline__ void open_step(const ModelDesc& md, int lb) {
+    if (lb == 0 && threadIdx.x == 0) count_step(md.F);
 }
 
-__device__ __forceinline__ void heat_flux_any(const ModelDesc& md, int lb) {
-    if (md.F.mat)
-        k_heat_flux_body<false>(md.m, md.F, md.cfg, lb);
-    else
-        k_heat_flux_body<true>(md.m, md.F, md.cfg, lb);
-}
-// a temperature model's first launch of a fused step: timeStep++,
-// currentTime += dt (once per model), then the heat flux
-__device__ __forceinline__ void heat_flux_opening_any(const ModelDesc& md, int lb) {
-    if (lb == 0 && threadIdx.x == 0) {
-        md.F.sc->time_step += 1;
-        md.F.sc->current_time += md.F.sc->dt;
+// One element tile: OP for a model of plugin P
+template <int OP, int P>
+__device__ __forceinline__ void elem_tile(TileSmem& S, const ModelDesc& md, int lb, bool temperature) {
+    if (OP == BOP_FUSED) {
+        open_step(md, lb);
+        if (temperature)
+            heat_flux_any(S, md, lb);
+        else
+            stress_any<P, true>(S, md, lb);
+    } else if (OP == BOP_FUSED_STRESS) {
+        stress_any<P, true>(S, md, lb);
+    } else if (OP == BOP_STRESS) {
+        stress_any<P, false>(S, md, lb);
+    } else {
+        heat_flux_any(S, md, lb);
     }
-    heat_flux_any(md, lb);
 }
 
 // Element-tile kernels: the fused end-of-step/next-stress kernel (or its
 // heat variant for models with temperature), the heat flux, the stress update.
 template <int OP>
-__global__ void __launch_bounds__(ELEM_WARPS * 32, SNAC_ELEM_MINB)
+__global__ void __launch_bounds__(ELEM_WARPS * 32, 4)
     kb_elements(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
     __shared__ ModelDesc md;
+    __shared__ __align__(16) TileSmem S;
     for (int i = blockIdx.x; i < ntiles; i += gridDim.x) {
         const int2 t = tiles[i];
         __syncthreads();  // the previous tile is done with md
         load_desc(md, D + t.x);
         __syncthreads();
-        const int P = md.cfg.constitutive;
-        if (OP == BOP_FUSED) {
-            if (md.cfg.temperature) {
-                heat_flux_opening_any(md, t.y);
-            } else {
-                switch (P) {
-                    case SNAC_RHEOLOGY_ELASTIC: fused_step_any<SNAC_RHEOLOGY_ELASTIC>(md, t.y); break;
-                    case SNAC_RHEOLOGY_PLASTIC: fused_step_any<SNAC_RHEOLOGY_PLASTIC>(md, t.y); break;
-                    case SNAC_RHEOLOGY_VISCOPLASTIC:
-                        fused_step_any<SNAC_RHEOLOGY_VISCOPLASTIC>(md, t.y);
-                        break;
-                    default: fused_step_any<SNAC_RHEOLOGY_MAXWELL>(md, t.y); break;
-                }
-            }
-        } else if (OP == BOP_FUSED_STRESS) {
-            switch (P) {
-                case SNAC_RHEOLOGY_ELASTIC: fused_step_any<SNAC_RHEOLOGY_ELASTIC>(md, t.y, false); break;
-                case SNAC_RHEOLOGY_PLASTIC: fused_step_any<SNAC_RHEOLOGY_PLASTIC>(md, t.y, false); break;
-                case SNAC_RHEOLOGY_VISCOPLASTIC:
-                    fused_step_any<SNAC_RHEOLOGY_VISCOPLASTIC>(md, t.y, false);
-                    break;
-                default: fused_step_any<SNAC_RHEOLOGY_MAXWELL>(md, t.y, false); break;
-            }
-        } else if (OP == BOP_STRESS) {
-            switch (P) {
-                case SNAC_RHEOLOGY_ELASTIC: calc_stresses_any<SNAC_RHEOLOGY_ELASTIC>(md, t.y); break;
-                case SNAC_RHEOLOGY_PLASTIC: calc_stresses_any<SNAC_RHEOLOGY_PLASTIC>(md, t.y); break;
-                case SNAC_RHEOLOGY_VISCOPLASTIC:
-                    calc_stresses_any<SNAC_RHEOLOGY_VISCOPLASTIC>(md, t.y);
-                    break;
-                default: calc_stresses_any<SNAC_RHEOLOGY_MAXWELL>(md, t.y); break;
-            }
-        } else {
-            heat_flux_any(md, t.y);
+        const bool temp = md.cfg.temperature != 0;
+        switch (md.cfg.constitutive) {
+            case SNAC_RHEOLOGY_ELASTIC: elem_tile<OP, SNAC_RHEOLOGY_ELASTIC>(S, md, t.y, temp); break;
+            case SNAC_RHEOLOGY_PLASTIC: elem_tile<OP, SNAC_RHEOLOGY_PLASTIC>(S, md, t.y, temp); break;
+            case SNAC_RHEOLOGY_VISCOPLASTIC: elem_tile<OP, SNAC_RHEOLOGY_VISCOPLASTIC>(S, md, t.y, temp); break;
+            default: elem_tile<OP, SNAC_RHEOLOGY_MAXWELL>(S, md, t.y, temp); break;
         }
     }
 }
@@ -138,26 +122,16 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32, SNAC_ELEM_MINB)
 // temperature on/off): the tile lists are grouped by class, and each class
 // present gets its own launch, without the run-time switch (fewer registers).
 template <int OP, int P, int TEMP>
-__global__ void __launch_bounds__(ELEM_WARPS * 32, SNAC_ELEM_MINB)
+__global__ void __launch_bounds__(ELEM_WARPS * 32, 4)
     kb_elements_c(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
     __shared__ ModelDesc md;
+    __shared__ __align__(16) TileSmem S;
     for (int i = blockIdx.x; i < ntiles; i += gridDim.x) {
         const int2 t = tiles[i];
         __syncthreads();
         load_desc(md, D + t.x);
         __syncthreads();
-        if (OP == BOP_FUSED) {
-            if (TEMP)
-                heat_flux_opening_any(md, t.y);
-            else
-                fused_step_any<P>(md, t.y);
-        } else if (OP == BOP_FUSED_STRESS) {
-            fused_step_any<P>(md, t.y, false);
-        } else if (OP == BOP_STRESS) {
-            calc_stresses_any<P>(md, t.y);
-        } else {
-            heat_flux_any(md, t.y);
-        }
+        elem_tile<OP, P>(S, md, t.y, TEMP != 0);
     }
 }
 
@@ -171,10 +145,17 @@ __host__ __device__ constexpr int plugin_slot(int constitutive) {
 
 // Node-tile kernels (one thread per node, or per element for the minimum
 // length scale); the block size is the tile size the tile list was built for.
+// The gathers have one stage (node_stage_bytes of dynamic shared memory).
+__host__ __device__ constexpr size_t node_stage_bytes(int op, int threads) {
+    return gather_stage_bytes(op == BOP_HEAT_NODES ? HEAT_CHUNK + HEAT_TAIL : 50, threads);
+}
 template <int OP>
 __global__ void __launch_bounds__(256) kb_nodes(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
     __shared__ ModelDesc md;
-    for (int i = blockIdx.x; i < ntiles; i += gridDim.x) {
+    __shared__ GatherSmem S;
+    if (OP != BOP_MINLS) gather_init(S);
+    unsigned phase = 0;
+    for (int i = blockIdx.x; i < ntiles; i += gridDim.x, phase ^= 1) {
         const int2 t = tiles[i];
         __syncthreads();
         load_desc(md, D + t.x);
@@ -182,18 +163,20 @@ __global__ void __launch_bounds__(256) kb_nodes(const ModelDesc* __restrict__ D,
         if (OP == BOP_LOOP_NODES) {
             const bool vo = md.cfg.vonly != 0;
             switch (md.cfg.dt_type) {
-                case SNAC_DT_CONSTANT: k_loop_nodes_body<SNAC_DT_CONSTANT, false>(md.m, md.F, md.cfg, t.y); break;
+                case SNAC_DT_CONSTANT:
+                    k_loop_nodes_body<SNAC_DT_CONSTANT, false>(S, md.m, md.F, md.cfg, t.y, 1, phase);
+                    break;
                 case SNAC_DT_DYNAMIC:
-                    if (vo) k_loop_nodes_body<SNAC_DT_DYNAMIC, true>(md.m, md.F, md.cfg, t.y);
-                    else k_loop_nodes_body<SNAC_DT_DYNAMIC, false>(md.m, md.F, md.cfg, t.y);
+                    if (vo) k_loop_nodes_body<SNAC_DT_DYNAMIC, true>(S, md.m, md.F, md.cfg, t.y, 1, phase);
+                    else k_loop_nodes_body<SNAC_DT_DYNAMIC, false>(S, md.m, md.F, md.cfg, t.y, 1, phase);
                     break;
                 default:
-                    if (vo) k_loop_nodes_body<SNAC_DT_WAVE, true>(md.m, md.F, md.cfg, t.y);
-                    else k_loop_nodes_body<SNAC_DT_WAVE, false>(md.m, md.F, md.cfg, t.y);
+                    if (vo) k_loop_nodes_body<SNAC_DT_WAVE, true>(S, md.m, md.F, md.cfg, t.y, 1, phase);
+                    else k_loop_nodes_body<SNAC_DT_WAVE, false>(S, md.m, md.F, md.cfg, t.y, 1, phase);
                     break;
             }
         } else if (OP == BOP_HEAT_NODES) {
-            k_heat_nodes_body(md.m, md.F, md.cfg, t.y);
+            k_heat_nodes_body(S, md.m, md.F, md.cfg, t.y, 1, phase);
         } else {
             k_min_length_scale_body(md.m, md.F, t.y);
         }

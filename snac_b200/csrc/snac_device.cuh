@@ -240,6 +240,30 @@ __host__ __device__ __forceinline__ double dvz(double x, double y, double z) {
 #endif
 }
 
+// The same window as one unsigned compare of a key, x != 0 only, so that a
+// group of operands costs two instructions each (the key and a running
+// maximum) and one compare; a group that fails it (a zero among its operands, mostly) is
+// looked at operand by operand with zero_or_within.
+template <int LO, int HI>
+__device__ __forceinline__ unsigned window_key(double x) {
+    return ((unsigned)__double2hiint(x) << 1) - ((unsigned)(1023 + LO) << 21);
+}
+template <int LO, int HI>
+__device__ __forceinline__ bool key_within(unsigned k) {
+    return k <= ((unsigned)(HI - LO + 1) << 21) - 1u;
+}
+template <int LO, int HI, int N>
+__device__ __forceinline__ bool all_zero_or_within(const double (&x)[N]) {
+    unsigned k = window_key<LO, HI>(x[0]);
+#pragma unroll
+    for (int i = 1; i < N; i++) k = max(k, window_key<LO, HI>(x[i]));
+    if (key_within<LO, HI>(k)) return true;
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < N; i++) ok = ok & zero_or_within<LO, HI>(x[i]);
+    return ok;
+}
+
 // Groups of quotients, in place: one window test and one branch for the
 // group instead of one per quotient (a branch per division splits the
 // instruction schedule); a group with any operand outside the window takes
@@ -248,13 +272,9 @@ template <int N>
 __host__ __device__ __forceinline__ void dvk_n(double (&x)[N], double c, double z) {
 #if defined(__CUDA_ARCH__) && SNAC_MARKSTEIN_DIV >= 1
     double q[N];
-    bool ok = true;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        q[i] = markstein(x[i], c, z, x[i] * z);
-        ok = ok & zero_or_within<-900, 900>(x[i]);
-    }
-    if (ok) {
+    for (int i = 0; i < N; i++) q[i] = markstein(x[i], c, z, x[i] * z);
+    if (all_zero_or_within<-900, 900>(x)) {
 #pragma unroll
         for (int i = 0; i < N; i++) x[i] = q[i];
     } else {
@@ -270,13 +290,9 @@ template <int N>
 __host__ __device__ __forceinline__ void dvz_n(double (&x)[N], double y, double z) {
 #if defined(__CUDA_ARCH__) && SNAC_MARKSTEIN_DIV >= 2
     double q[N];
-    bool ok = positive_within<-450, 450>(y);
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        q[i] = markstein(x[i], y, z, x[i] * z);
-        ok = ok & zero_or_within<-450, 450>(x[i]);
-    }
-    if (ok) {
+    for (int i = 0; i < N; i++) q[i] = markstein(x[i], y, z, x[i] * z);
+    if (positive_within<-450, 450>(y) && all_zero_or_within<-450, 450>(x)) {
 #pragma unroll
         for (int i = 0; i < N; i++) x[i] = q[i];
     } else {
@@ -340,6 +356,77 @@ __device__ __forceinline__ void tet_geometry(const V3 c[4], TetGeom& g) {
         tet_face(c[face_node(f, 0)], c[face_node(f, 1)], c[face_node(f, 2)], g.A[f], g.n[f]);
 }
 
+// ---- the same geometry for tame coordinates ------------------------------------------
+// A coordinate is tame when it is 0 or its magnitude lies in [2^-100, 2^140)
+// (a length in metres always does, short of an exact 0 that a wave front has
+// just begun to move).  Then nothing in a tet's geometry needs a range test
+// of its own:
+//   an edge component (a difference) is 0 or in [2^-152, 2^141]: both
+//     coordinates are multiples of 2^-152;
+//   a product of two is 0 or in [2^-304, 2^282], a multiple of 2^-356 or
+//     coarser after rounding, so a cross-product component is 0 or in
+//     [2^-357, 2^283];
+//   its square is 0 or in [2^-714, 2^566], a face's sum q of three in [2^-714, 2^568]
+//     unless all are 0, its root s in [2^-357, 2^284];
+//   the volume determinant is 0 or in [2^-562, 2^428].
+// So the quotients by 6 and by s lie inside the windows of dvk and dvz, and the root
+// and RN(1/s) come from one reciprocal-root seed.  A face with q = 0, a
+// volume outside [2^-450, 2^451) and a root whose low word is all ones (which
+// covers the one significand whose reciprocal the last step below may round wrongly) turn
+// `ok` off; the caller then takes the general form.
+constexpr int TAME_LO = -100, TAME_HI = 139;
+__device__ __forceinline__ bool tame_coordinate(double x) { return zero_or_within<TAME_LO, TAME_HI>(x); }
+// |x| < 2^140 (false for infinities and NaN)
+__device__ __forceinline__ bool tame_size(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) < ((unsigned)(1023 + TAME_HI + 1) << 20);
+}
+
+// s = RN(sqrt(q)) and z = RN(1/s) for q in [2^-714, 2^568]: Newton's coupled
+// iteration for sqrt(q) and 1/(2 sqrt(q)) from the hardware's approximate
+// reciprocal root (its error e goes to about 3/2 e^2 per pass: two passes
+// from 2^-20 reach rounding level), then Markstein's final steps, one FMA
+// each: s = RN(g + (q - g^2) h), and y + y (1 - s y) for the reciprocal,
+// which is RN(1/s) unless s has an all-ones significand (P. Markstein, IBM
+// J. Res. Dev. 34(1), 1990).  The device self-test compares both with the
+// IEEE root and quotient.
+__device__ __forceinline__ void sqrt_recip(double q, double& s, double& z) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+    double g = q * y, h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    s = fma(fma(-g, g, q), h, g);
+    y = h + h;
+    z = fma(fma(-s, y, 1.0), y, y);
+}
+
+__device__ __forceinline__ void tet_geometry_tame(const V3 c[4], TetGeom& g, bool& ok) {
+    const double x2 = c[1].x - c[0].x, y2 = c[1].y - c[0].y, z2 = c[1].z - c[0].z;
+    const double x3 = c[2].x - c[0].x, y3 = c[2].y - c[0].y, z3 = c[2].z - c[0].z;
+    const double x4 = c[3].x - c[0].x, y4 = c[3].y - c[0].y, z4 = c[3].z - c[0].z;
+    const double det = x4 * (y2 * z3 - z2 * y3) + y4 * (z2 * x3 - x2 * z3) + z4 * (x2 * y3 - x3 * y2);
+    g.V = fabs(markstein(det, 6.0, Z6, det * Z6));
+    g.zV = recip(g.V);
+    ok = ok & positive_within<-450, 450>(g.V);
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+        const V3 &c1 = c[face_node(f, 0)], &c2 = c[face_node(f, 1)], &c3 = c[face_node(f, 2)];
+        const double u2 = c2.x - c1.x, v2 = c2.y - c1.y, w2 = c2.z - c1.z;
+        const double u3 = c3.x - c1.x, v3 = c3.y - c1.y, w3 = c3.z - c1.z;
+        const double a = v2 * w3 - w2 * v3, b = w2 * u3 - u2 * w3, e = u2 * v3 - v2 * u3;
+        const double q = a * a + b * b + e * e;
+        double s, z;
+        sqrt_recip(q, s, z);
+        ok = ok & (__double2hiint(q) != 0) & (__double2loint(s) != -1);
+        g.A[f] = s * 0.5;
+        g.n[f] = {markstein(a, s, z, a * z), markstein(b, s, z, b * z), markstein(e, s, z, e * z)};
+    }
+}
+
 __device__ __forceinline__ double comp(const V3& v, int d) { return d == 0 ? v.x : (d == 1 ? v.y : v.z); }
 
 // sum_k w_k,a * n_face(k),b * A_face(k) over the tet's nodes k (node k pairs
@@ -367,37 +454,37 @@ __device__ __forceinline__ double shear_sum(const V3 v[4], const TetGeom& g, int
 
 // StrainRate.c:65-184, before the mixed-discretisation correction;
 // sr = (xx, yy, zz, xy, xz, yz)
-__device__ __forceinline__ void tet_strain_rate(const V3 v[4], const TetGeom& g, double sr[6]) {
+// tame: the tet's coordinates are tame, its velocities below 2^140 and its
+// volume in [2^-450, 2^451).  Then every sum is below 2^428, so the
+// quotient by 3 needs no range test (for the divisor 3 the correction step is
+// exact for every finite x: the remainder is a multiple of the smallest
+// subnormal, and x / 3 never lies halfway between two doubles), and the
+// quotient by V only the lower one.
+__device__ __forceinline__ void tet_strain_rate(const V3 v[4], const TetGeom& g, double sr[6], bool tame) {
     double t[6] = {-1.0f * (face_sum(v, 0, g, 0)), -1.0f * (face_sum(v, 1, g, 1)), -1.0f * (face_sum(v, 2, g, 2)),
                    -0.5f * (shear_sum(v, g, 0, 1)), -0.5f * (shear_sum(v, g, 0, 2)), -0.5f * (shear_sum(v, g, 1, 2))};
-    dvk_n(t, 3.0, Z3);
-    dvz_n(t, g.V, g.zV);
+    double u[6];
 #pragma unroll
-    for (int a = 0; a < 6; a++) sr[a] = t[a];
-}
-
-// spin rates r01, r02, r12 of a tet, UpdateElement.c:145-219
-__device__ __forceinline__ void spin_rates(const V3 v[4], const TetGeom& g, double (&r)[3]) {
-    // RN(0.5 / V) = 0.5 RN(1 / V) exactly while 1 / V is a normal number
-    const double hV = exp_within<-1000, 1000>(g.V) ? 0.5 * g.zV : ieee_div(0.5, g.V);
-    r[0] = -(hV) * (spin_sum(v, g, 0, 1));
-    r[1] = -(hV) * (spin_sum(v, g, 0, 2));
-    r[2] = -(hV) * (spin_sum(v, g, 1, 2));
-    dvk_n(r, 3.0, Z3);
+    for (int a = 0; a < 6; a++) {
+        u[a] = markstein(t[a], 3.0, Z3, t[a] * Z3);
+        sr[a] = markstein(u[a], g.V, g.zV, u[a] * g.zV);
+    }
+    if (!(tame && all_zero_or_within<-450, 450>(u))) {
+#pragma unroll
+        for (int a = 0; a < 6; a++) sr[a] = ieee_div(ieee_div(t[a], 3.0), g.V);
+    }
 }
 
 // The spin rates (UpdateElement.c:145-219) and the strain rate
-// (StrainRate.c:65-184) of one tet from the same velocities and geometry,
-// as the fused element kernel needs both: the chains
-// a0+a1+a2+a3 -/+ b0 -/+ b1 -/+ b2 -/+ b3 of a spin sum and of the matching
-// shear sum share their products and their prefix a0+..+a3, which are
-// formed once here; every result has the bits of spin_rates and
-// tet_strain_rate.
-__device__ __forceinline__ void spin_and_strain_rates(const V3 v[4], const TetGeom& g, double (&r)[3], double sr[6]) {
+// (StrainRate.c:65-184) of one tet from the same velocities and geometry:
+// the chains a0+a1+a2+a3 -/+ b0 -/+ b1 -/+ b2 -/+ b3 of a spin sum and of
+// the matching shear sum share their products and their prefix a0+..+a3,
+// formed once here; the bits of spin_rates and tet_strain_rate.
+__device__ __forceinline__ void spin_and_strain_rates(const V3 v[4], const TetGeom& g, double (&r)[3], double sr[6],
+                                                      bool tame) {
     double t[6];
-    t[0] = -1.0f * (face_sum(v, 0, g, 0));
-    t[1] = -1.0f * (face_sum(v, 1, g, 1));
-    t[2] = -1.0f * (face_sum(v, 2, g, 2));
+#pragma unroll
+    for (int k = 0; k < 3; k++) t[k] = -1.0f * (face_sum(v, k, g, k));
     constexpr int PA[3] = {0, 0, 1}, PB[3] = {1, 2, 2};
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -409,35 +496,47 @@ __device__ __forceinline__ void spin_and_strain_rates(const V3 v[4], const TetGe
         r[k] = pre - q0 - q1 - q2 - q3;
         t[3 + k] = -0.5f * (pre + q0 + q1 + q2 + q3);
     }
-    const double hV = exp_within<-1000, 1000>(g.V) ? 0.5 * g.zV : ieee_div(0.5, g.V);
+    // RN(0.5 / V) = 0.5 RN(1 / V) exactly while 1 / V is a normal number
+    const double hV = tame || exp_within<-1000, 1000>(g.V) ? 0.5 * g.zV : ieee_div(0.5, g.V);
 #pragma unroll
     for (int k = 0; k < 3; k++) r[k] = -(hV) * (r[k]);
-    dvk_n(r, 3.0, Z3);
-    dvk_n(t, 3.0, Z3);
-    dvz_n(t, g.V, g.zV);
+    double u[6];
 #pragma unroll
-    for (int a = 0; a < 6; a++) sr[a] = t[a];
+    for (int a = 0; a < 6; a++) {
+        u[a] = markstein(t[a], 3.0, Z3, t[a] * Z3);
+        sr[a] = markstein(u[a], g.V, g.zV, u[a] * g.zV);
+    }
+    if (!(tame && all_zero_or_within<-450, 450>(u))) {
+#pragma unroll
+        for (int a = 0; a < 6; a++) sr[a] = ieee_div(ieee_div(t[a], 3.0), g.V);
+    }
+    if (tame) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) r[a] = markstein(r[a], 3.0, Z3, r[a] * Z3);
+    } else {
+        dvk_n(r, 3.0, Z3);
+    }
+}
+
+// spin rates r01, r02, r12 of a tet, UpdateElement.c:145-219
+__device__ __forceinline__ void spin_rates(const V3 v[4], const TetGeom& g, double (&r)[3], bool tame) {
+    // RN(0.5 / V) = 0.5 RN(1 / V) exactly while 1 / V is a normal number
+    const double hV = tame || exp_within<-1000, 1000>(g.V) ? 0.5 * g.zV : ieee_div(0.5, g.V);
+    r[0] = -(hV) * (spin_sum(v, g, 0, 1));
+    r[1] = -(hV) * (spin_sum(v, g, 0, 2));
+    r[2] = -(hV) * (spin_sum(v, g, 1, 2));
+    if (tame) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) r[a] = markstein(r[a], 3.0, Z3, r[a] * Z3);
+    } else {
+        dvk_n(r, 3.0, Z3);
+    }
 }
 
 // Jaumann rotation of the stress with the spin rates r, UpdateElement.c:145-265
 // (the strain is zeroed first, :81, so its own rotation leaves it zero); s01
 // takes "+ r12*s02".
-__device__ __forceinline__ void rotate_stress_by(const double (&r)[3], double dt, double s[6]) {
-    const double r01 = r[0], r02 = r[1], r12 = r[2];
-    s[0] += (2.0f * r01 * s[3] + 2.0f * r02 * s[4]) * dt;
-    s[1] += (2.0f * (-1.0f * r01) * s[3] + 2.0f * r12 * s[5]) * dt;
-    s[2] += (2.0f * (-1.0f * r02) * s[4] + 2.0f * (-1.0f * r12) * s[5]) * dt;
-    s[3] += (r01 * (s[1] - s[0])) * dt + (r02 * s[5] + r12 * s[4]) * dt;
-    s[4] += (r02 * (s[2] - s[0])) * dt + (r01 * s[5] - r12 * s[3]) * dt;
-    s[5] += (r12 * (s[2] - s[1])) * dt + ((-1.0f * r01) * s[4] - r02 * s[3]) * dt;
-}
-
-// Jaumann rotation of the stress, UpdateElement.c:145-265 (the strain is
-// zeroed first, :81, so its own rotation leaves it zero); s01 takes "+ r12*s02".
-__device__ __forceinline__ void rotate_stress(const V3 v[4], const TetGeom& g, double dt, double s[6]) {
-    // RN(0.5 / V) = 0.5 RN(1 / V) exactly while 1 / V is a normal number
-    double r[3];
-    spin_rates(v, g, r);
+__device__ __forceinline__ void rotate_stress(const double (&r)[3], double dt, double s[6]) {
     const double r01 = r[0], r02 = r[1], r12 = r[2];
     s[0] += (2.0f * r01 * s[3] + 2.0f * r02 * s[4]) * dt;
     s[1] += (2.0f * (-1.0f * r01) * s[3] + 2.0f * r12 * s[5]) * dt;
@@ -577,8 +676,10 @@ __host__ __device__ __forceinline__ bool surely_elastic(const double st[6], doub
     double r0 = fabs(st[3]) + fabs(st[4]);
     double r1 = fabs(st[3]) + fabs(st[5]);
     double r2 = fabs(st[4]) + fabs(st[5]);
-    double hi = fmax(st[0] + r0, fmax(st[1] + r1, st[2] + r2));
-    double lo = fmin(st[0] - r0, fmin(st[1] - r1, st[2] - r2));
+    // (plain selects: with a NaN anywhere the tolerances are NaN and every test fails)
+    const double h0 = st[0] + r0, h1 = st[1] + r1, h2 = st[2] + r2, l0 = st[0] - r0, l1 = st[1] - r1, l2 = st[2] - r2;
+    const double h01 = h0 > h1 ? h0 : h1, l01 = l0 < l1 ? l0 : l1;
+    const double hi = h01 > h2 ? h01 : h2, lo = l01 < l2 ? l01 : l2;
     double scale = fabs(st[0]) + fabs(st[1]) + fabs(st[2]) + 2.0 * (r0 + r1 + r2);
     double cterm = 2.0 * cohesion * sqrt_anphi;
     double tol_t = 1e-9 * (scale + fabs(stc)) + 1e-300;
