@@ -109,6 +109,8 @@ struct snac_gpu {
     double* topo_scratch = nullptr;  // [nnx * nnz] topography-diffusion scratch
     OutputState* out = nullptr;
     HostStep* hs = nullptr;  // snac_gpu_step_host's streams and staging
+    void* adj_ws = nullptr;  // the adjoint's workspace, kept for the next call (see ADJ_KEEP)
+    size_t adj_ws_bytes = 0;
     // host mirror of the step bookkeeping
     int parity = 0;
     long long time_step = 0;
@@ -1168,7 +1170,7 @@ void snac_gpu_destroy(snac_gpu* h) {
     }
     void* bufs[] = {h->pos[0], h->pos[1], h->vel, h->force, h->stress, h->eps_p, h->pst, h->visc, h->density, h->vol,
                     h->hflux, h->tpre, h->fterm, h->bc, h->vbc_val, h->tbc_val, h->mat, h->mats, h->coh_scale, h->fric_scale,
-                    h->visc_scale, h->sc, h->stage, h->escal, h->residual_fr, h->topo_scratch};
+                    h->visc_scale, h->sc, h->stage, h->escal, h->residual_fr, h->topo_scratch, h->adj_ws};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (h->stream && h->own_stream) cudaStreamDestroy(h->stream);
@@ -2159,23 +2161,56 @@ struct Snap {
     long long time_step = 0;
 };
 
-int snap_alloc(snac_gpu* h, Snap& z) {
-    const long long nn = h->mesh.nn, nq = h->mesh.ne * NT;
-    int rc;
-    if ((rc = dalloc(h, &z.pos, nn)) || (rc = dalloc(h, &z.vel, nn)) || (rc = dalloc(h, &z.force, nn)) ||
-        (rc = dalloc(h, &z.stress, nq * 6)) || (rc = dalloc(h, &z.sc, 1)))
-        return rc;
-    // the hooks' own per-tet state: plastic strain (plastic, visco-plastic), volumes (Maxwell)
-    if (h->eps_p && (rc = dalloc(h, &z.eps_p, nq))) return rc;
-    if (h->vol && (rc = dalloc(h, &z.vol, nq * 2))) return rc;
+// The adjoint's buffers are carved from one allocation: a call needs some two
+// hundred (six or seven per kept state), whose separate allocation, clearing
+// and release took 35 of the 49 ms of a 60-step call at 16 k hexes.  Every
+// buffer is written before it is read.  A Carver without memory only counts.
+struct Carver {
+    char* base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T** p, long long n) {
+        if (base) *p = reinterpret_cast<T*>(base + used);
+        used += ((size_t)n * sizeof(T) + 255) & ~(size_t)255;
+    }
+};
+// the handle keeps a workspace up to this size between calls; a larger one is
+// released when its call ends
+constexpr size_t ADJ_KEEP = (size_t)512 << 20;
+
+int adj_ws_reserve(snac_gpu* h, size_t bytes) {
+    if (h->adj_ws_bytes >= bytes) return 0;
+    if (h->adj_ws) cudaFree(h->adj_ws);  // waits for whatever still uses it
+    h->alloc_bytes -= (long long)h->adj_ws_bytes;
+    h->adj_ws = nullptr;
+    h->adj_ws_bytes = 0;
+    cudaError_t e = cudaMalloc(&h->adj_ws, bytes);
+    if (e != cudaSuccess) {
+        h->adj_ws = nullptr;
+        return set_err(h, SNAC_GPU_ENOMEM, -1, "adjoint workspace: cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+    }
+    h->adj_ws_bytes = bytes;
+    h->alloc_bytes += (long long)bytes;
     return 0;
 }
+void adj_ws_trim(snac_gpu* h) {
+    if (h->adj_ws_bytes <= ADJ_KEEP) return;
+    cudaFree(h->adj_ws);
+    h->alloc_bytes -= (long long)h->adj_ws_bytes;
+    h->adj_ws = nullptr;
+    h->adj_ws_bytes = 0;
+}
 
-void snap_free(Snap& z) {
-    void* b[] = {z.pos, z.vel, z.force, z.stress, z.eps_p, z.sc, z.vol};
-    for (void* p : b)
-        if (p) cudaFree(p);
-    z = Snap();
+void snap_take(const snac_gpu* h, Carver& c, Snap& z) {
+    const long long nn = h->mesh.nn, nq = h->mesh.ne * NT;
+    c.take(&z.pos, nn);
+    c.take(&z.vel, nn);
+    c.take(&z.force, nn);
+    c.take(&z.stress, nq * 6);
+    c.take(&z.sc, 1);
+    // the hooks' own per-tet state: plastic strain (plastic, visco-plastic), volumes (Maxwell)
+    if (h->eps_p) c.take(&z.eps_p, nq);
+    if (h->vol) c.take(&z.vol, nq * 2);
 }
 
 // one launch copying the arrays of a state (sizes in 64-bit words)
@@ -2267,54 +2302,49 @@ int adj_nodes_launch(snac_gpu* h, const AdjState& cur, const AdjState& prev, con
     return launch_check_named(h, "k_adj_nodes");
 }
 
-int misfit(snac_gpu* h, const snac_adjoint_desc* a, const AdjBufs& B, double* terms_dev, double* loss) {
+struct AdjWork {
+    AdjBufs B{};
+    double* terms = nullptr;
+    double* targets = nullptr;  // [2][top nodes]: velocities, heights
+    double* grads = nullptr;    // [3][ne]
+};
+
+int misfit(snac_gpu* h, const snac_adjoint_desc* a, const AdjWork& w, double* loss) {
     const long long nt = (long long)h->mesh.nnx * h->mesh.nnz;
-    double *tv = nullptr, *ty = nullptr;
-    int rc;
-    if ((rc = dalloc(h, &tv, nt)) || (rc = dalloc(h, &ty, nt))) {
-        if (tv) cudaFree(tv);
-        return rc;
-    }
-    cudaMemcpyAsync(tv, a->target_vy, nt * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-    cudaMemcpyAsync(ty, a->target_y, nt * sizeof(double), cudaMemcpyHostToDevice, h->stream);
+    double *tv = w.targets, *ty = w.targets + nt;
+    CK(cudaMemcpyAsync(tv, a->target_vy, nt * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(ty, a->target_y, nt * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     k_adj_loss<<<(unsigned)((h->mesh.nn + 127) / 128), 128, 0, h->stream>>>(h->mesh, h->pos[h->parity], h->vel, tv, ty,
-                                                                          a->w_v, a->w_h, terms_dev, B);
+                                                                          a->w_v, a->w_h, w.terms, w.B);
     h->launches++;
-    rc = launch_check_named(h, "k_adj_loss");
-    std::vector<double> t(nt);
-    cudaError_t e = cudaMemcpyAsync(t.data(), terms_dev, nt * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(tv);
-    cudaFree(ty);
+    int rc = launch_check_named(h, "k_adj_loss");
     if (rc) return rc;
-    if (e != cudaSuccess) return set_err(h, SNAC_GPU_ECUDA, -1, "misfit: %s", cudaGetErrorString(e));
+    std::vector<double> t(nt);
+    CK(cudaMemcpyAsync(t.data(), w.terms, nt * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
     double L = 0.0;
     for (long long i = 0; i < nt; i++) L += t[i];
     *loss = L;
     return 0;
 }
 
-struct AdjWork {
-    AdjBufs B{};
-    double* terms = nullptr;
-    double* grads = nullptr;  // [3][ne]
-    void release() {
-        void* b[] = {B.xbar, B.vbar, B.fbar, B.cbuf, B.sbar, B.epbar, B.pbar, B.vobar, terms, grads};
-        for (void* p : b)
-            if (p) cudaFree(p);
-        *this = AdjWork();
-    }
-};
-
-int adj_work_alloc(snac_gpu* h, AdjWork& w) {
-    const long long nn = h->mesh.nn, nq = h->mesh.ne * NT, nt = (long long)h->mesh.nnx * h->mesh.nnz;
-    int rc;
-    if ((rc = dalloc(h, &w.B.xbar, nn)) || (rc = dalloc(h, &w.B.vbar, nn)) || (rc = dalloc(h, &w.B.fbar, nn)) ||
-        (rc = dalloc(h, &w.B.cbuf, h->mesh.ner * NT * 24)) || (rc = dalloc(h, &w.B.sbar, nq * 6)) || (rc = dalloc(h, &w.B.epbar, nq)) ||
-        (rc = dalloc(h, &w.B.pbar, nq * 3)) || (rc = dalloc(h, &w.terms, nt)) || (rc = dalloc(h, &w.grads, 3 * h->mesh.ne)))
-        return rc;
-    if (h->constitutive == SNAC_RHEOLOGY_MAXWELL && (rc = dalloc(h, &w.B.vobar, nq))) return rc;
-    return 0;
+void loss_take(const snac_gpu* h, Carver& c, AdjWork& w) {
+    const long long nn = h->mesh.nn, nt = (long long)h->mesh.nnx * h->mesh.nnz;
+    c.take(&w.B.xbar, nn);
+    c.take(&w.B.vbar, nn);
+    c.take(&w.B.fbar, nn);
+    c.take(&w.terms, nt);
+    c.take(&w.targets, 2 * nt);
+}
+void adj_work_take(const snac_gpu* h, Carver& c, AdjWork& w) {
+    const long long nq = h->mesh.ne * NT;
+    loss_take(h, c, w);
+    c.take(&w.B.cbuf, h->mesh.ner * NT * 24);
+    c.take(&w.B.sbar, nq * 6);
+    c.take(&w.B.epbar, nq);
+    c.take(&w.B.pbar, nq * 3);
+    c.take(&w.grads, 3 * h->mesh.ne);
+    if (h->constitutive == SNAC_RHEOLOGY_MAXWELL) c.take(&w.B.vobar, nq);
 }
 
 int adj_status(snac_gpu* h) {
@@ -2334,15 +2364,14 @@ extern "C" {
 int snac_gpu_misfit(snac_gpu* h, const snac_adjoint_desc* a, double* loss) {
     if (!h || !a || !loss || !a->target_vy || !a->target_y) return SNAC_GPU_EINVAL;
     AdjWork w;
-    int rc = 0;
-    const long long nn = h->mesh.nn, nt = (long long)h->mesh.nnx * h->mesh.nnz;
-    if ((rc = dalloc(h, &w.B.xbar, nn)) || (rc = dalloc(h, &w.B.vbar, nn)) || (rc = dalloc(h, &w.B.fbar, nn)) ||
-        (rc = dalloc(h, &w.terms, nt))) {
-        w.release();
-        return rc;
-    }
-    rc = misfit(h, a, w.B, w.terms, loss);
-    w.release();
+    Carver count, carve;
+    loss_take(h, count, w);
+    int rc = adj_ws_reserve(h, count.used);
+    if (rc) return rc;
+    carve.base = static_cast<char*>(h->adj_ws);
+    loss_take(h, carve, w);
+    rc = misfit(h, a, w, loss);
+    adj_ws_trim(h);
     return rc;
 }
 
@@ -2377,10 +2406,7 @@ int snac_gpu_adjoint_grads(snac_gpu* h, const snac_adjoint_desc* a, double* loss
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     auto cleanup = [&]() {
         cudaStreamSynchronize(h->stream);
-        for (auto& z : cp) snap_free(z);
-        for (auto& z : seg) snap_free(z);
-        snap_free(fin);
-        w.release();
+        adj_ws_trim(h);
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);
     };
@@ -2392,10 +2418,17 @@ int snac_gpu_adjoint_grads(snac_gpu* h, const snac_adjoint_desc* a, double* loss
             return rc_;     \
         }                   \
     } while (0)
-    for (auto& z : cp) ACK(snap_alloc(h, z));
-    for (auto& z : seg) ACK(snap_alloc(h, z));
-    ACK(snap_alloc(h, fin));
-    ACK(adj_work_alloc(h, w));
+    auto take_all = [&](Carver& c) {
+        for (auto& z : cp) snap_take(h, c, z);
+        for (auto& z : seg) snap_take(h, c, z);
+        snap_take(h, c, fin);
+        adj_work_take(h, c, w);
+    };
+    Carver count, carve;
+    take_all(count);
+    ACK(adj_ws_reserve(h, count.used));
+    carve.base = static_cast<char*>(h->adj_ws);
+    take_all(carve);
     for (auto& e : ev)
         if (cudaEventCreate(&e) != cudaSuccess) ACK(set_err(h, SNAC_GPU_ECUDA, -1, "cudaEventCreate"));
 
@@ -2409,7 +2442,7 @@ int snac_gpu_adjoint_grads(snac_gpu* h, const snac_adjoint_desc* a, double* loss
     ACK(snap_save(h, fin));
     cudaEventRecord(ev[1], h->stream);
     ACK(read_status(h));
-    ACK(misfit(h, a, w.B, w.terms, loss));  // also seeds the node adjoints
+    ACK(misfit(h, a, w, loss));  // also seeds the node adjoints
 
     // reverse sweep, segment by segment from the last
     const long long nq = h->mesh.ne * NT;
