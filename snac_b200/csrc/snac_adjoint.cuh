@@ -51,7 +51,8 @@ struct AdjBufs {
     double4* xbar;   // [nn] adjoint of x (w unused)
     double4* vbar;   // [nn] adjoint of v
     double4* fbar;   // [nn] adjoint of the damped-force input F (xyz) and of the inertial mass (w)
-    double* cbuf;    // per-tet corner adjoints (x 3, v 3) for the node gather: rows (t, corner, component) of ner hexes
+    double* cbuf;    // per-tet corner adjoints for the node gather: groups of CROWS rows, 4 chunks of
+                     // [6 components: x 3, v 3][10 corners] rows (as the force groups)
     double* sbar;    // [nq][6] adjoint of sigma_avg^{n-1}, handed to the next (earlier) step
     double* epbar;   // [nq] adjoint of eps_p
     double* pbar;    // [nq][3] adjoint of the cohesion, friction, viscosity scales
@@ -65,8 +66,13 @@ __device__ __forceinline__ D3 d3(double x, double y, double z) { return {x, y, z
 __device__ __forceinline__ D3 operator-(D3 a, D3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ D3 operator+(D3 a, D3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ D3 operator*(double s, D3 a) { return {s * a.x, s * a.y, s * a.z}; }
-__device__ __forceinline__ D3 cross(D3 a, D3 b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
-__device__ __forceinline__ double dot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// the reverse sweep needs no reference rounding: fused multiply-adds
+__device__ __forceinline__ D3 cross(D3 a, D3 b) {
+    return {fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x))};
+}
+__device__ __forceinline__ double dot(D3 a, D3 b) { return fma(a.x, b.x, fma(a.y, b.y, a.z * b.z)); }
+__device__ __forceinline__ D3 fma3(double s, D3 a, D3 b) { return {fma(s, a.x, b.x), fma(s, a.y, b.y), fma(s, a.z, b.z)}; }
+constexpr int CCHUNK = 60, CROWS = 4 * CCHUNK;
 __device__ __forceinline__ double cmp(const D3& a, int d) { return d == 0 ? a.x : (d == 1 ? a.y : a.z); }
 __device__ __forceinline__ void addc(D3& a, int d, double v) {
     if (d == 0) a.x += v;
@@ -75,9 +81,6 @@ __device__ __forceinline__ void addc(D3& a, int d, double v) {
 }
 __device__ __forceinline__ double sgnd(double x) { return x < 0 ? -1.0 : (x > 0 ? 1.0 : 0.0); }
 
-#ifndef SNAC_ADJ_SMEM_REC
-#define SNAC_ADJ_SMEM_REC 1  // the forward record in shared memory (fewer spills; measured faster)
-#endif
 // ---- forward record of the constitutive update of one tet --------------------------------
 struct ConsRec {
     // visco-plastic Maxwell step
@@ -189,35 +192,45 @@ __device__ __forceinline__ void mc_reverse(const ConsRec& R, const double sb_out
     sb_in[5] = S[1][2] + S[2][1];
 }
 
+// Shared memory of the reverse kernel: the triples and hex sums of the
+// forward, the forward records, the block's group of corner adjoints
+struct AdjSmem {
+    Triple tri[ELEM_WARPS];
+    TripleCoords fbar[ELEM_WARPS];
+    double hex_terms[ELEM_WARPS][2][3 * 12];
+    double rows[CROWS * GROUP];
+    ConsRec rec[ELEM_WARPS * 32];
+};
+
 // ---- the per-tet reverse kernel ------------------------------------------------------------
 template <int PLUGIN>
-__device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, const Config& cfg, const AdjState& S,
+__device__ __forceinline__ void adj_tet_body(AdjSmem& sm, const Mesh& m, const Fields& F, const Config& cfg, const AdjState& S,
                                              const AdjBufs& B, int rotate, int first_rev, double dt, int lb) {
     // hooks with a Mohr-Coulomb return map and a plastic strain
     constexpr bool MC = PLUGIN == SNAC_RHEOLOGY_PLASTIC || PLUGIN == SNAC_RHEOLOGY_VISCOPLASTIC;
-    TetSlot s = tet_slot(m, lb);
-    // corners of step n
-    V3 c[4], v[4];
-    double T[4];
-    long long nid[4];
-#pragma unroll
-    for (int qn = 0; qn < 4; qn++) {
-        if (s.active) {
-            nid[qn] = corner_node(m, s.i, s.j, s.k, tet_node_rt(s.t, qn));
-            double4 p = S.pos[nid[qn]];
-            double4 w = S.vel[nid[qn]];
-            c[qn] = {p.x, p.y, p.z};
-            T[qn] = p.w;
-            v[qn] = {w.x, w.y, w.z};
-        } else {
-            nid[qn] = 0;
-            c[qn] = {qn == 1 ? 1.0 : 0.0, qn == 2 ? 1.0 : 0.0, qn == 3 ? 1.0 : 0.0};
-            v[qn] = {0.0, 0.0, 0.0};
-            T[qn] = 0.0;
-        }
+    // the triple of step n's state, fetched as the forward fetches it
+    Triple& z = sm.tri[threadIdx.x >> 5];
+    TripleCoords& zf = sm.fbar[threadIdx.x >> 5];
+    {
+        Fields FS = F;
+        FS.pos = S.pos;
+        FS.vel = const_cast<double4*>(S.vel);
+        FS.stress = const_cast<double*>(S.stress);
+        FS.eps_p = const_cast<double*>(S.eps_p);
+        fetch_triple<stress_need(PLUGIN)>(m, FS, lb, z);
+        FS.pos = B.fbar;  // and the nodes' force adjoints, the same way
+        fetch_triple<0>(m, FS, lb, zf);
     }
+    const TetLane L = tet_lane();
+    const TetSlot s = tet_slot_of(m, L, lb);
+    const unsigned slots = TET_SLOTS[s.t];
+    cp_async_wait_all();
+    __syncwarp();
+    const TetView<Triple> view{z, L.rows};
     TetGeom g;
-    tet_geometry(c, g);
+    const bool tame = triple_geometry<true>(z, L, g);
+    V3 v[4];
+    view.velocities(v);
     // area vectors w_f = n_f A_f (= half the face cross product)
     D3 w[4];
 #pragma unroll
@@ -228,11 +241,8 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     for (int k = 0; k < 4; k++) vk[k] = d3(v[k].x, v[k].y, v[k].z);
 
     // ---------------- forward recompute --------------------------------------------------
-    double s_in[6] = {0, 0, 0, 0, 0, 0};
-    if (s.active) {
-#pragma unroll
-        for (int a = 0; a < 6; a++) s_in[a] = S.stress[s.q * 6 + a];
-    }
+    double s_in[6];
+    stage_stress(s, z, s_in);
     double s_pre[6];
 #pragma unroll
     for (int a = 0; a < 6; a++) s_pre[a] = s_in[a];
@@ -240,7 +250,7 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     double r01 = 0, r02 = 0, r12 = 0;
     if (rotate) {
         double r[3];
-        spin_rates(v, g, r, false);
+        spin_rates(v, g, r, tame);
         rotate_stress(r, dt, s_pre);
         r01 = r[0];
         r02 = r[1];
@@ -250,18 +260,19 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     for (int a = 0; a < 6; a++) s_mid[a] = s_pre[a];
 
     double sr[6];
-    tet_strain_rate(v, g, sr, false);
+    tet_strain_rate(v, g, sr, tame);
     double sr_raw[6];
 #pragma unroll
     for (int a = 0; a < 6; a++) sr_raw[a] = sr[a];
-    const double vsum = grp_sum(g.V, s.base);
+    const double tr1 = dv3(sr[0] + sr[1] + sr[2]);
+    double(&hx)[2][3 * 12] = sm.hex_terms[threadIdx.x >> 5];
+    hex_put(hx[0], s.lane, s.base, s.t, g.V);
+    hex_put(hx[1], s.lane, s.base, s.t, tr1 * g.V);
+    __syncwarp();
+    const double vsum = hex_total(hx[0], s.base);
+    const double P1 = hex_total(hx[1], s.base);
     const double VS = 2.0 * (vsum * 0.5);
     const double zVS = recip(VS);
-    const double tr1 = dv3(sr[0] + sr[1] + sr[2]);
-    const double tr1V = tr1 * g.V;  // the term formed on its own lane, as the forward does
-    double P1 = 0.0f;
-#pragma unroll
-    for (int u = 0; u < NT; u++) P1 += grp(tr1V, s.base, u);
     const double corr1 = -1.0f * tr1 + dvz(P1, VS, zVS);
     sr[0] += corr1;
     sr[1] += corr1;
@@ -270,22 +281,15 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
 #pragma unroll
     for (int a = 0; a < 6; a++) e[a] = sr[a] * dt;
 
-    const int ph = s.active ? phase_of(F, s.e) : 0;
+    const int ph = phase_of(F, s.e);
     const DevMaterial& M = F.mats[ph];
-    const double cs = (F.coh_scale && s.active) ? F.coh_scale[s.e] : 1.0;
-    const double fsc = (F.fric_scale && s.active) ? F.fric_scale[s.e] : 1.0;
-    const double vsc = (F.visc_scale && s.active) ? F.visc_scale[s.e] : 1.0;
-    double eps_p = (MC && s.active) ? S.eps_p[s.q] : 0.0;
-    const double eps_p0 = eps_p;
+    const TetIn in = load_tet_in<PLUGIN>(F, s, z);
+    const double cs = MC ? in.coh : 1.0, fsc = MC ? in.fric : 1.0, vsc = MC ? in.visc : 1.0;
+    double eps_p = in.eps_p;
 
-#if SNAC_ADJ_SMEM_REC
-    // the record lives in shared memory (dynamic, one per thread): its ~50
-    // doubles then hold no registers between the forward and the reverse
-    extern __shared__ __align__(16) unsigned char adj_smem[];
-    ConsRec& R = reinterpret_cast<ConsRec*>(adj_smem)[threadIdx.x];
-#else
-    ConsRec R;
-#endif
+    // the record lives in shared memory, one per thread: its ~50 doubles then
+    // hold no registers between the forward and the reverse
+    ConsRec& R = sm.rec[threadIdx.x];
     double st[6];
 #pragma unroll
     for (int a = 0; a < 6; a++) st[a] = s_pre[a];
@@ -307,8 +311,8 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
         // includes the shear strains, and only phase 0 takes the update
         R.mx = (ph == 0);
         R.trs = st[0] + st[1] + st[2];
-        R.vcur = rotate ? g.V : (s.active ? S.vol[s.q * 2 + 0] : 1.0);
-        R.vold = s.active ? S.vol[s.q * 2 + (rotate ? 0 : 1)] : 1.0;
+        R.vcur = rotate ? g.V : S.vol[s.q * 2 + 0];
+        R.vold = S.vol[s.q * 2 + (rotate ? 0 : 1)];
         R.tre = dv(R.vcur, R.vold) - 1.0f;
         const double tn3 = dv3(R.tre), ts3 = dv3(R.trs);
         for (int a = 0; a < 3; a++) R.d[a] = e[a] - tn3;
@@ -319,7 +323,7 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
         if (J == 0.0f) J = M.refsrate;
         R.J = J;
         double avgTemp = 0.0;
-        for (int qn = 0; qn < 4; qn++) avgTemp += 0.25 * T[qn];
+        for (int qn = 0; qn < 4; qn++) avgTemp += 0.25 * view.T(qn);
         const double eta = arrhenius_viscosity(M, M.refvisc, J, avgTemp);
         R.eta_free = (eta > M.vis_min && eta < M.vis_max);
         R.eta = eta;
@@ -344,11 +348,14 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
         if (J == 0.0f) J = M.refsrate;
         R.J = J;
         double avgTemp = 0.0;
-        for (int qn = 0; qn < 4; qn++) avgTemp += 0.25 * T[qn];
+        for (int qn = 0; qn < 4; qn++) avgTemp += 0.25 * view.T(qn);
         const double refvisc = M.refvisc * vsc;
         // unclipped viscosity without the element's scale: d eta / d scale
-        R.eta_base = arrhenius_base(M, M.refvisc, J, avgTemp);
-        double eta = arrhenius_viscosity(M, refvisc, J, avgTemp);
+        const double ex = arrhenius_base(M, 1.0, J, avgTemp);
+        R.eta_base = M.refvisc * ex;
+        double eta = refvisc * ex;  // as arrhenius_viscosity forms it
+        if (eta < M.vis_min) eta = M.vis_min;
+        if (eta > M.vis_max) eta = M.vis_max;
         R.eta_free = (eta > M.vis_min && eta < M.vis_max);
         R.eta = eta;
         R.tmp = dv(M.mu, 2.0f * (eta)) * dt;
@@ -360,113 +367,101 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     const double a1 = M.lambda + 2.0f * M.mu;
     const double a2 = M.lambda;
     R.yield = false;
-    R.tension = false;
-    R.alam = 0.0;
-    R.inc = 0.0;
-    R.co = R.hd = R.fa = R.da = R.fa_b = R.co_b = R.tgf_b = R.tgc_b = R.tgd = 0.0;
-    R.sphi = R.spsi = R.anphi = R.anpsi = R.stc = 0.0;
-    R.dpl = 1.0;
-    R.clamped = false;
-    R.stc_from_co = false;
     if (MC) {
-        // softening lookup: this tet's own segment (plastic: first match, clamp past the end;
-        // visco-plastic: last match)
-        bool matched = false;
+        // softening lookup: this tet's own segment (plastic: first match, clamp past the
+        // end; visco-plastic: last match), the scales applied to the table
+        // entries exactly as the forward does, for identical branch decisions
+        int seg = -1;
+        bool past = false;
         for (int i = 0; i < M.nsegments; i++) {
-            const double pl1 = M.plstrain[i];
             const double pl2 = M.plstrain[i + 1];
-            if (eps_p >= pl1 && eps_p <= pl2) {
-                const double dpl = pl2 - pl1;
-                R.dpl = dpl;
-                double tg[3] = {M.fric[i + 1] - M.fric[i], M.coh[i + 1] - M.coh[i], M.dil[i + 1] - M.dil[i]};
-                dvz_n(tg, dpl, M.zpl[i]);
-                R.tgf_b = tg[0];
-                R.tgc_b = tg[1];
-                R.tgd = tg[2];
-                R.fa_b = M.fric[i] + R.tgf_b * (eps_p - pl1);
-                R.co_b = M.coh[i] + R.tgc_b * (eps_p - pl1);
-                R.da = M.dil[i] + R.tgd * (eps_p - pl1);
-                matched = true;
-                R.clamped = false;
+            if (eps_p >= M.plstrain[i] && eps_p <= pl2) {
+                seg = i;
                 if (PLUGIN == SNAC_RHEOLOGY_PLASTIC) break;
             } else if (PLUGIN == SNAC_RHEOLOGY_PLASTIC && i == M.nsegments - 1 && eps_p > pl2) {
-                R.fa_b = M.fric[M.nsegments];
-                R.co_b = M.coh[M.nsegments];
-                R.da = M.dil[M.nsegments];
-                R.tgf_b = R.tgc_b = R.tgd = 0.0;
-                matched = true;
-                R.clamped = true;
+                past = true;
                 break;
             }
         }
-        if (s.active && !matched) report(F.sc, SNAC_GPU_ENOTSUP, s.e);  // the carried-over lookup is not differentiated
-        // values as the forward forms them (scales applied to the table entries)
-        {
-            // recompute exactly as the forward does, for identical branch decisions
-            double fa = 0.0, co = 0.0, hd = 0.0;
-            for (int i = 0; i < M.nsegments; i++) {
-                const double pl1 = M.plstrain[i];
-                const double pl2 = M.plstrain[i + 1];
-                double f0 = F.fric_scale ? M.fric[i] * fsc : M.fric[i];
-                double f1 = F.fric_scale ? M.fric[i + 1] * fsc : M.fric[i + 1];
-                double c0 = F.coh_scale ? M.coh[i] * cs : M.coh[i];
-                double c1 = F.coh_scale ? M.coh[i + 1] * cs : M.coh[i + 1];
-                if (eps_p >= pl1 && eps_p <= pl2) {
-                    double tg[2] = {f1 - f0, c1 - c0};
-                    dvz_n(tg, pl2 - pl1, M.zpl[i]);
-                    const double tgf = tg[0], tgc = tg[1];
-                    fa = f0 + tgf * (eps_p - pl1);
-                    co = c0 + tgc * (eps_p - pl1);
-                    hd = tgc;
-                    if (PLUGIN == SNAC_RHEOLOGY_PLASTIC) break;
-                } else if (PLUGIN == SNAC_RHEOLOGY_PLASTIC && i == M.nsegments - 1 && eps_p > pl2) {
-                    fa = F.fric_scale ? M.fric[M.nsegments] * fsc : M.fric[M.nsegments];
-                    co = F.coh_scale ? M.coh[M.nsegments] * cs : M.coh[M.nsegments];
-                    hd = 0.0;
-                    break;
-                }
+        R.clamped = past;
+        if (s.active && seg < 0 && !past) report(F.sc, SNAC_GPU_ENOTSUP, s.e);  // the carried-over lookup is not differentiated
+        const bool angles_const = M.fric_const && M.dil_const;
+        double fa = 0.0, co = 0.0, hd = 0.0, da = 0.0;
+        if (seg >= 0) {
+            const double dep = eps_p - M.plstrain[seg], dpl = M.plstrain[seg + 1] - M.plstrain[seg], zpl = M.zpl[seg];
+            const double c0 = M.coh[seg] * cs;
+            hd = dvz(M.coh[seg + 1] * cs - c0, dpl, zpl);
+            co = c0 + hd * dep;
+            fa = M.fric0;
+            da = M.dil0;
+            if (!angles_const) {
+                const double f0 = M.fric[seg] * fsc;
+                double tg[2] = {M.fric[seg + 1] * fsc - f0, M.dil[seg + 1] - M.dil[seg]};
+                dvz_n(tg, dpl, zpl);
+                fa = f0 + tg[0] * dep;
+                da = M.dil[seg] + tg[1] * dep;
             }
-            R.fa = fa;
-            R.co = co;
-            R.hd = hd;
+        } else if (past) {
+            fa = M.fric[M.nsegments] * fsc;
+            co = M.coh[M.nsegments] * cs;
+            da = M.dil[M.nsegments];
         }
-        const bool phi_ok = (PLUGIN == SNAC_RHEOLOGY_PLASTIC) ? (R.fa >= 0.0f) : (R.fa > 0.0f);
+        R.fa = fa;
+        R.co = co;
+        R.hd = hd;
+        R.da = da;
+        const bool phi_ok = (PLUGIN == SNAC_RHEOLOGY_PLASTIC) ? (fa >= 0.0f) : (fa > 0.0f);
         if (s.active && !phi_ok) report(F.sc, SNAC_GPU_ENOTSUP, s.e);
-        R.stc = M.ten_off;
-        R.stc_from_co = false;
+        double stc = M.ten_off;
+        bool stc_from_co = false;
         // constant-angle values as the forward takes them (host-evaluated, same bits)
-        const bool fconst = M.fric_const && R.fa == M.fric0;
-        if (R.fa > 0.0) {
-            double tmp = fconst ? dvz(R.co, M.tan_fric0, M.ztan_fric0) : dv(R.co, tan_fric(M, R.fa));
-            if (tmp < R.stc) {
-                R.stc = tmp;
-                R.stc_from_co = true;
+        const bool fconst = M.fric_const && fa == M.fric0;
+        if (fa > 0.0) {
+            double tmp = fconst ? dvz(co, M.tan_fric0, M.ztan_fric0) : dv(co, tan_fric(M, fa));
+            if (tmp < stc) {
+                stc = tmp;
+                stc_from_co = true;
             }
         }
-        R.sphi = sin_fric(M, R.fa);
-        R.spsi = sin_dil(M, R.da);
-        R.anphi = fconst ? M.anphi0 : dv(1.0f + R.sphi, 1.0f - R.sphi);
-        R.anpsi = (M.dil_const && R.da == M.dil0) ? M.anpsi0 : dv(1.0f + R.spsi, 1.0f - R.spsi);
-        double st_trial[6];
-#pragma unroll
-        for (int a = 0; a < 6; a++) st_trial[a] = st[a];
-        if (!surely_elastic(st, R.co, R.anphi, fconst ? M.sq_anphi0 : sqrt(R.anphi), R.stc)) {
+        const bool dconst = M.dil_const && da == M.dil0;
+        const double sphi = fconst ? M.sin_fric0 : sin_fric(M, fa), spsi = dconst ? M.sin_dil0 : sin_dil(M, da);
+        const double anphi = fconst ? M.anphi0 : dv(1.0f + sphi, 1.0f - sphi);
+        const double anpsi = dconst ? M.anpsi0 : dv(1.0f + spsi, 1.0f - spsi);
+        if (!surely_elastic(st, co, anphi, fconst ? M.sq_anphi0 : sqrt(anphi), stc)) {
+            R.stc = stc;
+            R.stc_from_co = stc_from_co;
+            R.sphi = sphi;
+            R.spsi = spsi;
+            R.anphi = anphi;
+            R.anpsi = anpsi;
+            // the table without the scales: d / d scale and d / d eps_p
+            if (seg >= 0) {
+                const double dep = eps_p - M.plstrain[seg], dpl = M.plstrain[seg + 1] - M.plstrain[seg];
+                double tg[3] = {M.fric[seg + 1] - M.fric[seg], M.coh[seg + 1] - M.coh[seg], M.dil[seg + 1] - M.dil[seg]};
+                dvz_n(tg, dpl, M.zpl[seg]);
+                R.tgf_b = tg[0];
+                R.tgc_b = tg[1];
+                R.tgd = tg[2];
+                R.fa_b = M.fric[seg] + tg[0] * dep;
+                R.co_b = M.coh[seg] + tg[1] * dep;
+            } else {
+                R.fa_b = past ? M.fric[M.nsegments] : 0.0;
+                R.co_b = past ? M.coh[M.nsegments] : 0.0;
+                R.tgf_b = R.tgc_b = R.tgd = 0.0;
+            }
             principal_stresses(st, R.sp, R.cn);
             double sp[3] = {R.sp[0], R.sp[1], R.sp[2]};
-            double fs = sp[0] - sp[2] * R.anphi + 2 * R.co * sqrt(R.anphi);
-            double ft = sp[2] - R.stc;
-            double aP = sqrt(1.0f + R.anphi * R.anphi) + R.anphi;
-            double sP = R.stc * R.anphi - 2 * R.co * sqrt(R.anphi);
-            double hh = sp[2] - R.stc + aP * (sp[0] - sP);
+            double fs = sp[0] - sp[2] * anphi + 2 * co * sqrt(anphi);
+            double ft = sp[2] - stc;
+            double aP = sqrt(1.0f + anphi * anphi) + anphi;
+            double sP = stc * anphi - 2 * co * sqrt(anphi);
+            double hh = sp[2] - stc + aP * (sp[0] - sP);
             R.tension = !(hh < 0.0f);
             const double ep_before = eps_p;
-            R.yield = mc_return_map(sp, R.cn, st, eps_p, R.co, R.hd, R.anphi, R.anpsi, R.stc, a1, a2) != 0;
-            (void)fs;
-            (void)ft;
+            R.yield = mc_return_map(sp, R.cn, st, eps_p, co, hd, anphi, anpsi, stc, a1, a2) != 0;
             if (R.yield) {
                 R.alam = R.tension ? dv(ft, a1)
-                                   : dv(fs, a1 - a2 * R.anpsi + a1 * R.anphi * R.anpsi - a2 * R.anphi +
-                                                2.0 * sqrt(R.anphi) * R.hd);
+                                   : dv(fs, a1 - a2 * anpsi + a1 * anphi * anpsi - a2 * anphi + 2.0 * sqrt(anphi) * hd);
                 R.inc = eps_p - ep_before;
                 for (int k = 0; k < 3; k++) R.sq[k] = sp[k];
             }
@@ -474,10 +469,10 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     }
     // stress averaging over the hex
     const double trS = dv3(st[0] + st[1] + st[2]);
-    const double trSV = trS * g.V;
-    double P2 = 0.0f;
-#pragma unroll
-    for (int u = 0; u < NT; u++) P2 += grp(trSV, s.base, u);
+    __syncwarp();  // every lane has read the volumes
+    hex_put(hx[0], s.lane, s.base, s.t, trS * g.V);
+    __syncwarp();
+    const double P2 = hex_total(hx[0], s.base);
     const double corr2 = -1.0f * trS + dvz(P2, VS, zVS);
     double sa[6];
 #pragma unroll
@@ -490,36 +485,51 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     // The reverse sweep needs no reference rounding: divisions by constants and
     // by the tet volume are multiplications by reciprocals.
     constexpr double K16 = 1.0 / 6.0, K13 = 1.0 / 3.0;
+    // sum over the hex's tets (lanes past the mesh repeat its last hex and store nothing)
+    auto reverse_sum = [&](double x) {
+        __syncwarp();
+        hex_put(hx[1], s.lane, s.base, s.t, x);
+        __syncwarp();
+        return hex_total(hx[1], s.base);
+    };
     const double iVS = zVS, i9V = (1.0 / 9.0) * g.zV, i3V = K13 * g.zV, i6V = K16 * g.zV;
     D3 wb[4] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     D3 vb[4] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     double Vb = 0.0;
     double sab[6] = {0, 0, 0, 0, 0, 0};
-    if (s.active && !first_rev) {
+    if (!first_rev) {
+        const double2* sbar = reinterpret_cast<const double2*>(B.sbar + s.q * 6);
 #pragma unroll
-        for (int a = 0; a < 6; a++) sab[a] = B.sbar[s.q * 6 + a];
+        for (int a = 0; a < 3; a++) {
+            const double2 x = sbar[a];
+            sab[2 * a] = x.x;
+            sab[2 * a + 1] = x.y;
+        }
     }
     // Force: node k takes sigma . w_{(k+1)%4} / 6, -g rho V / 8 in y, and the inertial mass
     // of face (k+1)%4 (constant dt: (lambda + 2 mu) max_d w_d^2 / (9 V) dt^2)
     const double rho = M.density;
     const double alpha1 = (M.lambda + 2.0f * M.mu);
-    if (s.active) {
+    {
+        const double vg = -cfg.gravity * rho / 8.0, m9 = alpha1 * i9V * (dt * dt);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int f = (k + 1) & 3;
-            const double4 fb = B.fbar[nid[k]];
+            const double2 fxy = zf.node[view.row(k)], fzw = zf.node[TripleCoords::PART + view.row(k)];
+            const double4 fb = make_double4(fxy.x, fxy.y, fzw.x, fzw.y);
             const D3& wf = w[f];
-            sab[0] += fb.x * wf.x * K16;
-            sab[1] += fb.y * wf.y * K16;
-            sab[2] += fb.z * wf.z * K16;
-            sab[3] += (fb.x * wf.y + fb.y * wf.x) * K16;
-            sab[4] += (fb.x * wf.z + fb.z * wf.x) * K16;
-            sab[5] += (fb.y * wf.z + fb.z * wf.y) * K16;
-            wb[f].x += (sa[0] * fb.x + sa[3] * fb.y + sa[4] * fb.z) * K16;
-            wb[f].y += (sa[3] * fb.x + sa[1] * fb.y + sa[5] * fb.z) * K16;
-            wb[f].z += (sa[4] * fb.x + sa[5] * fb.y + sa[2] * fb.z) * K16;
-            Vb += -cfg.gravity * rho / 8.0 * fb.y;
-            // inertial mass of face f
+            const D3 b6 = d3(fb.x * K16, fb.y * K16, fb.z * K16);
+            sab[0] = fma(b6.x, wf.x, sab[0]);
+            sab[1] = fma(b6.y, wf.y, sab[1]);
+            sab[2] = fma(b6.z, wf.z, sab[2]);
+            sab[3] = fma(b6.x, wf.y, fma(b6.y, wf.x, sab[3]));
+            sab[4] = fma(b6.x, wf.z, fma(b6.z, wf.x, sab[4]));
+            sab[5] = fma(b6.y, wf.z, fma(b6.z, wf.y, sab[5]));
+            wb[f].x = fma(sa[0], b6.x, fma(sa[3], b6.y, sa[4] * b6.z));
+            wb[f].y = fma(sa[3], b6.x, fma(sa[1], b6.y, sa[5] * b6.z));
+            wb[f].z = fma(sa[4], b6.x, fma(sa[5], b6.y, sa[2] * b6.z));
+            Vb = fma(vg, fb.y, Vb);
+            // inertial mass of face f: its largest component, the first of equals
             int dstar = 0;
             double best = wf.x * wf.x;
             if (wf.y * wf.y > best) {
@@ -530,9 +540,9 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
                 best = wf.z * wf.z;
                 dstar = 2;
             }
-            const double mf = alpha1 * best * i9V * (dt * dt);
-            addc(wb[f], dstar, fb.w * alpha1 * 2.0 * cmp(wf, dstar) * i9V * (dt * dt));
-            Vb += -fb.w * mf * g.zV;
+            const double fm = fb.w * m9;
+            addc(wb[f], dstar, fm * 2.0 * cmp(wf, dstar));
+            Vb = fma(-fm * best, g.zV, Vb);
         }
     }
     // trace averaging: sa_dd = st_dd - trS + P2 / VS
@@ -541,8 +551,8 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     for (int a = 0; a < 6; a++) stb[a] = sab[a];
     const double c2b = sab[0] + sab[1] + sab[2];
     const double P2b_own = c2b * iVS;  // summed over the hex below
-    const double P2b = grp_sum(s.active ? P2b_own : 0.0, s.base);
-    double VSb = -(P2 * (iVS * iVS)) * grp_sum(s.active ? c2b : 0.0, s.base);
+    const double P2b = reverse_sum(P2b_own);
+    double VSb = -(P2 * iVS) * P2b;
     double trSb = -c2b + P2b * g.V;
     Vb += P2b * trS;
     stb[0] += trSb * K13;
@@ -550,7 +560,7 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     stb[2] += trSb * K13;
 
     // constitutive reverse: MC return map
-    double epb = (s.active && !first_rev) ? B.epbar[s.q] : 0.0;  // adjoint of eps_p^{n+1}
+    double epb = !first_rev ? B.epbar[s.q] : 0.0;  // adjoint of eps_p^{n+1}
     double cob = 0.0, hdb = 0.0, anphib = 0.0, anpsib = 0.0, stcb = 0.0;
     double trialb[6];
     if (R.yield) {
@@ -560,24 +570,24 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
         for (int a = 0; a < 6; a++) trialb[a] = stb[a];
     }
     // softening chain: anphi(sphi(fa)), anpsi(spsi(da)), stc(co, fa)
-    const double deg = degrad();
-    double fab = 0.0, dab = 0.0;
-    if (MC) {
+    double csb = 0.0, fscb = 0.0;
+    if (MC && R.yield) {
+        const double deg = degrad();
         const double dan = 2.0 / ((1.0 - R.sphi) * (1.0 - R.sphi));
-        fab += anphib * dan * cos(R.fa * deg) * deg;
+        double fab = anphib * dan * cos(R.fa * deg) * deg;
         const double dap = 2.0 / ((1.0 - R.spsi) * (1.0 - R.spsi));
-        dab += anpsib * dap * cos(R.da * deg) * deg;
+        const double dab = anpsib * dap * cos(R.da * deg) * deg;
         if (R.stc_from_co) {
             const double tn = tan(R.fa * deg);
             const double cs2 = cos(R.fa * deg);
             cob += stcb / tn;
             fab += stcb * (-R.co / (tn * tn)) * (deg / (cs2 * cs2));
         }
+        // co = cs * co_b(eps_p), hd = cs * tgc_b, fa = fsc * fa_b(eps_p), da(eps_p)
+        csb = cob * R.co_b + hdb * R.tgc_b;
+        fscb = fab * R.fa_b;
+        epb += cob * cs * R.tgc_b + fab * fsc * R.tgf_b + dab * R.tgd;
     }
-    // co = cs * co_b(eps_p), hd = cs * tgc_b, fa = fsc * fa_b(eps_p), da(eps_p)
-    double csb = cob * R.co_b + hdb * R.tgc_b;
-    double fscb = fab * R.fa_b;
-    epb += cob * cs * R.tgc_b + fab * fsc * R.tgf_b + dab * R.tgd;
     double vscb = 0.0;
 
     // elastic trial (plastic), elastic update, or Maxwell step (Maxwell, visco-plastic)
@@ -687,30 +697,23 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
 #pragma unroll
     for (int a = 0; a < 6; a++) srb[a] = eb[a] * dt;
     const double c1b = srb[0] + srb[1] + srb[2];
-    const double P1b = grp_sum(s.active ? c1b * iVS : 0.0, s.base);
-    VSb += -(P1 * (iVS * iVS)) * grp_sum(s.active ? c1b : 0.0, s.base);
+    const double P1b = reverse_sum(c1b * iVS);
+    VSb = fma(-(P1 * iVS), P1b, VSb);
     const double tr1b = -c1b + P1b * g.V;
     Vb += P1b * tr1;
     srb[0] += tr1b * K13;
     srb[1] += tr1b * K13;
     srb[2] += tr1b * K13;
     // raw strain rate: sr_d = -S_dd / (3V), sr_ab = -(S_ab + S_ba) / (6V), S_ab = sum_k v_k,a w_k,b
+    double Sb[3][3];
+    for (int d = 0; d < 3; d++) Sb[d][d] = -srb[d] * i3V;
+    Sb[0][1] = Sb[1][0] = -srb[3] * i6V;
+    Sb[0][2] = Sb[2][0] = -srb[4] * i6V;
+    Sb[1][2] = Sb[2][1] = -srb[5] * i6V;
     {
-        double Sb[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        for (int d = 0; d < 3; d++) Sb[d][d] = -srb[d] * i3V;
-        Sb[0][1] = Sb[1][0] = -srb[3] * i6V;
-        Sb[0][2] = Sb[2][0] = -srb[4] * i6V;
-        Sb[1][2] = Sb[2][1] = -srb[5] * i6V;
-        for (int a = 0; a < 6; a++) Vb += srb[a] * (-sr_raw[a] * g.zV);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const D3& wk = w[(k + 1) & 3];
-            for (int a = 0; a < 3; a++)
-                for (int b = 0; b < 3; b++) {
-                    addc(vb[k], a, Sb[a][b] * cmp(wk, b));
-                    addc(wb[(k + 1) & 3], b, Sb[a][b] * cmp(vk[k], a));
-                }
-        }
+        double acc = 0.0;
+        for (int a = 0; a < 6; a++) acc = fma(srb[a], sr_raw[a], acc);
+        Vb = fma(-acc, g.zV, Vb);
     }
     // rotation of step n-1: s_pre = Rot(s_in, r, dt), in place, in the forward's order
     double sinb[6];
@@ -761,22 +764,27 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
         b[4] += 2.0 * dt * r02 * b[0];
         r01b += 2.0 * dt * si[3] * b[0];
         r02b += 2.0 * dt * si[4] * b[0];
-        // r_ab = -SP_ab / (6 V), SP_ab = sum_k (v_k,a w_k,b - v_k,b w_k,a)
+        // r_ab = -SP_ab / (6 V), SP_ab = S_ab - S_ba
         const double rr[3] = {r01, r02, r12};
         const double rb[3] = {r01b, r02b, r12b};
         const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
         for (int r = 0; r < 3; r++) {
             const double SPb = -rb[r] * i6V;
-            Vb += rb[r] * (-rr[r] * g.zV);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const D3& wk = w[(k + 1) & 3];
-                addc(vb[k], pa[r], SPb * cmp(wk, pb[r]));
-                addc(vb[k], pb[r], -SPb * cmp(wk, pa[r]));
-                addc(wb[(k + 1) & 3], pb[r], SPb * cmp(vk[k], pa[r]));
-                addc(wb[(k + 1) & 3], pa[r], -SPb * cmp(vk[k], pb[r]));
-            }
+            Vb = fma(rb[r] * -rr[r], g.zV, Vb);
+            Sb[pa[r]][pb[r]] += SPb;
+            Sb[pb[r]][pa[r]] -= SPb;
         }
+    }
+    // the adjoint of S_ab = sum_k v_k,a w_k,b, from the strain and the spin rates together
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int f = (k + 1) & 3;
+        const D3& wk = w[f];
+        const D3& vv = vk[k];
+        vb[k] = d3(dot(d3(Sb[0][0], Sb[0][1], Sb[0][2]), wk), dot(d3(Sb[1][0], Sb[1][1], Sb[1][2]), wk),
+                   dot(d3(Sb[2][0], Sb[2][1], Sb[2][2]), wk));
+        wb[f] = wb[f] + d3(dot(d3(Sb[0][0], Sb[1][0], Sb[2][0]), vv), dot(d3(Sb[0][1], Sb[1][1], Sb[2][1]), vv),
+                           dot(d3(Sb[0][2], Sb[1][2], Sb[2][2]), vv));
     }
     // VS = sum over the hex of V; VSb already holds the hex total (both terms
     // were summed over the hex), so every tet's V receives it once
@@ -790,8 +798,12 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
     // geometry: V = |det(c1-c0, c2-c0, c3-c0)| / 6, w_f = ((c_f1 - c_f0) x (c_f2 - c_f0)) / 2
     D3 cb[4] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     D3 C[4];
+    {
+        V3 c[4];
+        view.coords(c);
 #pragma unroll
-    for (int k = 0; k < 4; k++) C[k] = d3(c[k].x, c[k].y, c[k].z);
+        for (int k = 0; k < 4; k++) C[k] = d3(c[k].x, c[k].y, c[k].z);
+    }
     {
         const D3 x2 = C[1] - C[0], x3 = C[2] - C[0], x4 = C[3] - C[0];
         const double det = dot(x4, cross(x2, x3));
@@ -813,30 +825,37 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
         cb[f0] = cb[f0] - (ub + vvb);
     }
 
-    if (s.active) {
-        // tet-major rows, as the forward's force terms: the node gather reads
-        // one row at consecutive hexes
-        const long long R = m.ner;
-        double* o = B.cbuf + (long long)(s.t * 24) * R + s.e;
+    if (s.lane < 30) {
+        double* const r = sm.rows + (threadIdx.x >> 5) * 3 + s.base / 10;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            o[(k * 6 + 0) * R] = cb[k].x;
-            o[(k * 6 + 1) * R] = cb[k].y;
-            o[(k * 6 + 2) * R] = cb[k].z;
-            o[(k * 6 + 3) * R] = vb[k].x;
-            o[(k * 6 + 4) * R] = vb[k].y;
-            o[(k * 6 + 5) * R] = vb[k].z;
+            double* const o = r + corner_row(slots, (k + 1) & 3, CCHUNK);
+            o[0] = cb[k].x;
+            o[ROW10] = cb[k].y;
+            o[2 * ROW10] = cb[k].z;
+            o[3 * ROW10] = vb[k].x;
+            o[4 * ROW10] = vb[k].y;
+            o[5 * ROW10] = vb[k].z;
         }
+    }
+    if (s.active) {
         // pass 0 leaves the adjoint of the stress the state held
+        double2* sbar = reinterpret_cast<double2*>(B.sbar + s.q * 6);
 #pragma unroll
-        for (int a = 0; a < 6; a++) B.sbar[s.q * 6 + a] = sinb[a];
+        for (int a = 0; a < 3; a++) sbar[a] = make_double2(sinb[2 * a], sinb[2 * a + 1]);
         if (PLUGIN == SNAC_RHEOLOGY_MAXWELL) B.vobar[s.q] = rotate ? Vob : 0.0;
         B.epbar[s.q] = epb;
-        B.pbar[s.q * 3 + 0] += csb;
-        B.pbar[s.q * 3 + 1] += fscb;
-        B.pbar[s.q * 3 + 2] += vscb;
+        // a tet that adds nothing leaves its sums as they are
+        if (csb != 0.0) B.pbar[s.q * 3 + 0] += csb;
+        if (fscb != 0.0) B.pbar[s.q * 3 + 1] += fscb;
+        if (vscb != 0.0) B.pbar[s.q * 3 + 2] += vscb;
     }
-    (void)eps_p0;
+    bulk_fence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bulk_store(B.cbuf + (long long)lb * (CROWS * GROUP), sm.rows, CROWS * GROUP * 8);
+        bulk_drain();
+    }
 }
 
 #ifndef SNAC_ADJ_MINB
@@ -845,7 +864,8 @@ __device__ __forceinline__ void adj_tet_body(const Mesh& m, const Fields& F, con
 template <int PLUGIN>
 __global__ void __launch_bounds__(ELEM_WARPS * 32, SNAC_ADJ_MINB) k_adj_tet(Mesh m, Fields F, Config cfg, AdjState S, AdjBufs B,
                                                              int rotate, int first_rev, double dt) {
-    adj_tet_body<PLUGIN>(m, F, cfg, S, B, rotate, first_rev, dt, blockIdx.x);
+    extern __shared__ __align__(16) unsigned char g_gather[];
+    adj_tet_body<PLUGIN>(*reinterpret_cast<AdjSmem*>(g_gather), m, F, cfg, S, B, rotate, first_rev, dt, blockIdx.x);
 }
 
 // Node adjoints: gather the corner adjoints of tet pass n (fixed order), then
@@ -853,32 +873,36 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32, SNAC_ADJ_MINB) k_adj_tet(Mesh
 //   x^n = x^{n-1} + dt v^n,  v^n_c = v^{n-1}_c + dt F_d,c / m  (free components)
 //   F_d = F (1 - demf sgn(v^{n-1}) sgn(F))
 // cur = S^n (its force holds F_d and m of step n-1), prev = S^{n-1} (velocities).
-__global__ void __launch_bounds__(128) k_adj_nodes(Mesh m, Fields F, AdjState cur, AdjState prev, AdjBufs B,
-                                                   int gather, int update, double dt, double demf) {
-    long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= m.nn) return;
-    double4 xb = B.xbar[n], vb = B.vbar[n];
-    if (gather) {
-        int i, j, k;
-        split3(n, m.nnx, m.nny, i, j, k);
-        for (int ne = 0; ne < 8; ne++) {
-            int ei = i - 1 + (ne & 1), ej = j - 1 + ((ne >> 1) & 1), ek = k - 1 + ((ne >> 2) & 1);
-            if (ei < 0 || ej < 0 || ek < 0 || ei >= m.nx || ej >= m.ny || ek >= m.nz) continue;
-            long long e = (long long)ei + (long long)ej * m.nx + (long long)ek * m.nx * m.ny;
-            for (int idx = 0; idx < 5; idx++) {
-                const int t = node_tet(ne, idx);
-                const int qn = (node_face(ne, idx) + 3) & 3;  // face f is opposite local node (f+3)%4
-                const long long R = m.ner;
-                const double* o = B.cbuf + (long long)(t * 24 + qn * 6) * R + e;
-                xb.x += o[0];
-                xb.y += o[R];
-                xb.z += o[2 * R];
-                vb.x += o[3 * R];
-                vb.y += o[4 * R];
-                vb.z += o[5 * R];
-            }
-        }
+__global__ void __launch_bounds__(NODE_THREADS) k_adj_nodes(Mesh m, Fields F, AdjState cur, AdjState prev, AdjBufs B,
+                                                           int gather, int update, double dt, double demf, int stages) {
+    __shared__ GatherSmem S;
+    const int n = blockIdx.x * NODE_THREADS + threadIdx.x;
+    const bool active = n < (int)m.nn;
+    double4 xb = make_double4(0.0, 0.0, 0.0, 0.0), vb = xb;
+    if (active) {
+        xb = B.xbar[n];
+        vb = B.vbar[n];
     }
+    if (gather) {
+        gather_init(S);
+        int i = 0, j = 0, k = 0;
+        if (active) split3(n, m.nnx, m.nny, i, j, k);
+        const Gather<CCHUNK, 0> G{S, B.cbuf, CROWS, stages, gather_groups(NODE_THREADS) * CCHUNK * GROUP, 0};
+        const bool ok = G.run(m, blockIdx.x, active, i, j, k, [&](int ne, const double* r) {
+#pragma unroll
+            for (int idx = 0; idx < 5; idx++) {
+                const double* const o = r + pair_slot(ne, idx) * GROUP;
+                xb.x += o[0];
+                xb.y += o[ROW10];
+                xb.z += o[2 * ROW10];
+                vb.x += o[3 * ROW10];
+                vb.y += o[4 * ROW10];
+                vb.z += o[5 * ROW10];
+            }
+        });
+        if (!ok) report(F.sc, SNAC_GPU_ETIMEDOUT, n);
+    }
+    if (!active) return;
     if (update) {
         vb.x += dt * xb.x;
         vb.y += dt * xb.y;

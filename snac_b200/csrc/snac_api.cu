@@ -264,8 +264,9 @@ Fields fields(const snac_gpu* h) { return fields_at(h, h->parity); }
 unsigned elem_blocks(const Mesh& m) { return (unsigned)((m.ne + ELEM_PER_BLOCK - 1) / ELEM_PER_BLOCK); }
 
 // The launch of a node gather over blocks of NODE_THREADS nodes; rows: of a
-// stage.  As many stages as the grid leaves shared memory for: four (107 KB
-// of a momentum gather) up to two blocks per SM, two up to four, else one.
+// stage.  As many stages as let every block of the grid be resident at once
+// (227 KB of shared memory per SM, of which a block takes 1 KB besides), else one:
+// a grid of more than one wave hides a pair's latency behind its other blocks.
 struct NodeLaunch {
     unsigned blocks;
     int stages;
@@ -274,9 +275,10 @@ struct NodeLaunch {
 NodeLaunch node_launch(const snac_gpu* h, unsigned blocks, int rows) {
     NodeLaunch l;
     l.blocks = blocks;
-    const unsigned sms = (unsigned)h->n_sm;
-    l.stages = blocks <= 2 * sms ? 4 : blocks <= 4 * sms ? 2 : 1;
-    l.smem = (size_t)l.stages * gather_stage_bytes(rows, NODE_THREADS);
+    const size_t stage = gather_stage_bytes(rows, NODE_THREADS);
+    for (l.stages = 4; l.stages > 1; l.stages /= 2)
+        if (blocks <= (227u << 10) / (l.stages * stage + 1024) * (unsigned)h->n_sm) break;
+    l.smem = (size_t)l.stages * stage;
     return l;
 }
 unsigned node_blocks(const Mesh& m) { return (unsigned)((m.nn + NODE_THREADS - 1) / NODE_THREADS); }
@@ -904,7 +906,6 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
     m.nnz = d->nz + 1;
     m.ne = (long long)d->nx * d->ny * d->nz;
     m.nn = (long long)m.nnx * m.nny * m.nnz;
-    m.ner = (m.ne + 3) & ~3LL;
     h->constitutive = d->constitutive;
     h->temperature = d->temperature;
     h->abi = d_in->abi_version;
@@ -2273,10 +2274,9 @@ int adjoint_supported(snac_gpu* h) {
 template <int P>
 int adj_tet_launch_p(snac_gpu* h, const Fields& F, const AdjState& S, const AdjBufs& B, int rotate, int first_rev,
                      double dt) {
-    const size_t smem = SNAC_ADJ_SMEM_REC ? (size_t)ELEM_WARPS * 32 * sizeof(ConsRec) : 0;
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_adj_tet<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_adj_tet<P><<<elem_blocks(h->mesh), ELEM_WARPS * 32, smem, h->stream>>>(h->mesh, F, h->cfg, S, B, rotate, first_rev,
-                                                                              dt);
+    CK(allow_smem(k_adj_tet<P>, sizeof(AdjSmem)));
+    k_adj_tet<P><<<elem_blocks(h->mesh), ELEM_WARPS * 32, sizeof(AdjSmem), h->stream>>>(h->mesh, F, h->cfg, S, B, rotate,
+                                                                                       first_rev, dt);
     return 0;
 }
 
@@ -2296,8 +2296,10 @@ int adj_tet_launch(snac_gpu* h, const AdjState& S, const AdjBufs& B, int rotate,
 
 int adj_nodes_launch(snac_gpu* h, const AdjState& cur, const AdjState& prev, const AdjBufs& B, int gather, int update,
                      double dt) {
-    k_adj_nodes<<<(unsigned)((h->mesh.nn + 127) / 128), 128, 0, h->stream>>>(h->mesh, fields(h), cur, prev, B, gather,
-                                                                           update, dt, h->cfg.demf);
+    const NodeLaunch l = node_launch(h, node_blocks(h->mesh), CCHUNK);
+    CK(allow_smem(k_adj_nodes, l.smem));
+    k_adj_nodes<<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, fields(h), cur, prev, B, gather, update, dt,
+                                                              h->cfg.demf, l.stages);
     h->launches++;
     return launch_check_named(h, "k_adj_nodes");
 }
@@ -2339,7 +2341,7 @@ void loss_take(const snac_gpu* h, Carver& c, AdjWork& w) {
 void adj_work_take(const snac_gpu* h, Carver& c, AdjWork& w) {
     const long long nq = h->mesh.ne * NT;
     loss_take(h, c, w);
-    c.take(&w.B.cbuf, h->mesh.ner * NT * 24);
+    c.take(&w.B.cbuf, (h->mesh.ne + GROUP - 1) / GROUP * CROWS * GROUP);
     c.take(&w.B.sbar, nq * 6);
     c.take(&w.B.epbar, nq);
     c.take(&w.B.pbar, nq * 3);

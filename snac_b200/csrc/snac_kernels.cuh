@@ -35,7 +35,6 @@ namespace snac {
 struct Mesh {
     int nx, ny, nz, nnx, nny, nnz;
     long long ne, nn;
-    long long ner;  // row length of the tet-major adjoint arrays: ne rounded up to 4 (32-byte rows)
     int frows;      // rows of a force group: 130 (Config::vonly), 140, or 170 (constant dt)
 };
 
@@ -224,29 +223,7 @@ struct TetSlot {
     int lane, base, t;
     long long e, q;
     bool active;
-    int i, j, k;
 };
-
-__device__ __forceinline__ TetSlot tet_slot(const Mesh& m, int lb) {
-    TetSlot s;
-    s.lane = threadIdx.x & 31;
-    int g = s.lane / 10;
-    s.base = g * 10;
-    s.t = s.lane - s.base;
-    long long warp = (long long)lb * ELEM_WARPS + (threadIdx.x >> 5);
-    s.e = warp * 3 + g;
-    s.active = (g < 3) && (s.e < m.ne);
-    if (g >= 3) {  // lanes 30, 31 mirror lane 0-9 group 0 slots so shuffles stay in range
-        s.base = 0;
-        s.t = s.lane - 30;
-    }
-    s.q = s.e * NT + s.t;
-    if (s.active)
-        elem_ijk(m, s.e, s.i, s.j, s.k);
-    else
-        s.i = s.j = s.k = 0;
-    return s;
-}
 
 // ---- element blocks ---------------------------------------------------------------------
 // A block takes GROUP consecutive hexes, each of its warps a triple of them:
@@ -372,7 +349,6 @@ __device__ __forceinline__ TetSlot tet_slot_of(const Mesh& m, const TetLane& L, 
     s.active = L.lane < 30 && e < m.ne;
     s.e = e < m.ne ? e : m.ne - 1;
     s.q = s.e * NT + s.t;
-    s.i = s.j = s.k = 0;
     return s;
 }
 
@@ -1335,7 +1311,7 @@ struct Gather {
             const double* g = src + (long long)(S.g0[c] + lane) * (frows * GROUP);
             double* d = stage(c) + lane * (ROWS * GROUP);
             bulk_load(d, g + c * (CHUNK * GROUP), CHUNK * GROUP * 8, bar);
-            bulk_load(d + CHUNK * GROUP, g + 4 * (CHUNK * GROUP), TAIL * GROUP * 8, bar);
+            if (TAIL > 0) bulk_load(d + CHUNK * GROUP, g + 4 * (CHUNK * GROUP), TAIL * GROUP * 8, bar);
         }
     }
     static __device__ __forceinline__ void bulk_load(double* d, const double* s, unsigned bytes, unsigned bar) {
