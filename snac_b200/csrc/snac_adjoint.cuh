@@ -451,17 +451,18 @@ __device__ __forceinline__ void adj_tet_body(AdjSmem& sm, const Mesh& m, const F
             }
             principal_stresses(st, R.sp, R.cn);
             double sp[3] = {R.sp[0], R.sp[1], R.sp[2]};
-            double fs = sp[0] - sp[2] * anphi + 2 * co * sqrt(anphi);
+            const double sq_anphi = fconst ? M.sq_anphi0 : sqrt(anphi);
+            double fs = sp[0] - sp[2] * anphi + 2 * co * sq_anphi;
             double ft = sp[2] - stc;
-            double aP = sqrt(1.0f + anphi * anphi) + anphi;
-            double sP = stc * anphi - 2 * co * sqrt(anphi);
+            const double aP = fconst ? M.ap0 : sqrt(1.0f + anphi * anphi) + anphi;
+            double sP = stc * anphi - 2 * co * sq_anphi;
             double hh = sp[2] - stc + aP * (sp[0] - sP);
             R.tension = !(hh < 0.0f);
             const double ep_before = eps_p;
-            R.yield = mc_return_map(sp, R.cn, st, eps_p, co, hd, anphi, anpsi, stc, a1, a2) != 0;
+            R.yield = mc_return_map(sp, R.cn, st, eps_p, co, hd, anphi, sq_anphi, aP, anpsi, stc, a1, a2) != 0;
             if (R.yield) {
                 R.alam = R.tension ? dv(ft, a1)
-                                   : dv(fs, a1 - a2 * anpsi + a1 * anphi * anpsi - a2 * anphi + 2.0 * sqrt(anphi) * hd);
+                                   : dv(fs, a1 - a2 * anpsi + a1 * anphi * anpsi - a2 * anphi + 2.0 * sq_anphi * hd);
                 R.inc = eps_p - ep_before;
                 for (int k = 0; k < 3; k++) R.sq[k] = sp[k];
             }

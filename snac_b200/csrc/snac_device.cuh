@@ -88,7 +88,7 @@ struct DevMaterial {
     // constant angle, (1 + sin)/(1 - sin) of friction and dilation,
     // sqrt of the former and RN(1 / tan(friction))
     double zpl[SNAC_MAX_SEGMENTS];
-    double anphi0, anpsi0, sq_anphi0, ztan_fric0;
+    double anphi0, anpsi0, sq_anphi0, ap0, ztan_fric0;  // ap0 = sqrt(1 + anphi0^2) + anphi0
     // host-evaluated transcendentals (valid when the *_const flag is set)
     int fric_const, dil_const;
     double fric0, sin_fric0, tan_fric0;
@@ -404,6 +404,16 @@ __device__ __forceinline__ void sqrt_recip(double q, double& s, double& z) {
     z = fma(fma(-s, y, 1.0), y, y);
 }
 
+// z = RN(1/y) for y in [1, 2^64] whose low word is not all ones: Newton from
+// the hardware's approximate reciprocal, the last step Markstein's (see sqrt_recip).
+__device__ __forceinline__ double recip_mid(double y) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+    r = fma(fma(-y, r, 1.0), r, r);
+    r = fma(fma(-y, r, 1.0), r, r);
+    return fma(fma(-y, r, 1.0), r, r);
+}
+
 __device__ __forceinline__ void tet_geometry_tame(const V3 c[4], TetGeom& g, bool& ok) {
     const double x2 = c[1].x - c[0].x, y2 = c[1].y - c[0].y, z2 = c[1].z - c[0].z;
     const double x3 = c[2].x - c[0].x, y3 = c[2].y - c[0].y, z3 = c[2].z - c[0].z;
@@ -551,7 +561,7 @@ __device__ __forceinline__ void rotate_stress(const double (&r)[3], double dt, d
 // (most compressive first) and their directions cn[k] = eigenvector k.
 // The three (ip,iq) pairs and their rotate loops are spelled out so that the
 // whole solver lives in registers.
-__host__ __device__ __forceinline__ void jrot(double& aij, double& akl, double s, double tau) {
+__device__ __forceinline__ void jrot(double& aij, double& akl, double s, double tau) {
     double g = aij, h = akl;
     aij = g - s * (h + g * tau);
     akl = h + s * (g - h * tau);
@@ -563,25 +573,39 @@ struct Jac {
     double v[3][3];
 };
 
+// The rotation of one pair.  Its quotients and roots are correctly rounded, as
+// the reference's, but only the first needs the general division:
+// 1 + theta^2 lies in [1, 2^121] (|h| < 100 2^54 |apq| in that branch), |t| <= 1, so
+// 1 + t^2 in [1, 2] and 1 + c in [1.7, 2].  The operands that the short forms round
+// wrongly (an all-ones significand, as 1 + c has for t near 2^-26; a
+// subnormal range) take the IEEE division.
 template <int IP, int IQ>
-__host__ __device__ __forceinline__ void jac_pair(Jac& J, int i, double tresh) {
+__device__ __forceinline__ void jac_pair(Jac& J, int i, double tresh) {
     double& apq = (IP == 0 && IQ == 1) ? J.a01 : (IP == 0 && IQ == 2) ? J.a02 : J.a12;
     double g = 100.0f * fabs(apq);
     if ((i > 4) && (double)(fabs(J.d[IP]) + g) == (double)fabs(J.d[IP]) &&
         (double)(fabs(J.d[IQ]) + g) == (double)fabs(J.d[IQ])) {
         apq = 0.0f;
     } else if (fabs(apq) > tresh) {
-        double h = J.d[IQ] - J.d[IP], t;
-        if ((fabs(h) + g) == fabs(h)) {
-            t = dv(apq, h);
-        } else {
-            double theta = dv(0.5f * h, apq);
-            t = dv(1.0f, fabs(theta) + sqrt(1.0f + theta * theta));
+        double h = J.d[IQ] - J.d[IP];
+        const bool far = (fabs(h) + g) == fabs(h);
+        // t = apq / h, or theta = h / 2 / apq
+        double t = dv(far ? apq : 0.5f * h, far ? h : apq);
+        if (!far) {
+            const double theta = t, q = 1.0f + theta * theta;
+            double root, unused;
+            sqrt_recip(q, root, unused);
+            const double y = fabs(theta) + root;
+            t = recip_mid(y);
+            if (__double2loint(y) == -1) t = ieee_div(1.0, y);
             if (theta < 0.0f) t *= -1.0f;
         }
-        double c = dv(1.0f, sqrt(1.0f + t * t));
+        double root, c;
+        sqrt_recip(1.0f + t * t, root, c);
         double s = t * c;
-        double tau = dv(s, 1.0f + c);
+        const double y = 1.0f + c, zy = recip_mid(y);
+        double tau = markstein(s, y, zy, s * zy);
+        if (__double2loint(y) == -1 || !zero_or_within<-450, 450>(s)) tau = ieee_div(s, y);
         h = t * apq;
         J.z[IP] -= h;
         J.z[IQ] += h;
@@ -597,7 +621,7 @@ __host__ __device__ __forceinline__ void jac_pair(Jac& J, int i, double tresh) {
     }
 }
 
-__host__ __device__ void principal_stresses(const double st[6], double sp[3], double cn[3][3]) {
+__device__ __forceinline__ void principal_stresses(const double st[6], double sp[3], double cn[3][3]) {
     Jac J;
     J.a01 = st[3];
     J.a02 = st[4];
@@ -774,19 +798,19 @@ __device__ __noinline__ bool dp_return_map(double s[6], double sd[3], const doub
 
 // Mohr-Coulomb composite yield + return map in principal space, shared by
 // plastic/Constitutive.c:180-237 and viscoplastic/Constitutive.c:305-370.
+// sq_anphi = sqrt(anphi), aP = sqrt(1 + anphi^2) + anphi.
 // Returns 1 when the tet yielded (stress resolved back, plastic strain grown).
 __device__ __forceinline__ int mc_return_map(double sp[3], const double cn[3][3], double st6[6], double& eps_p,
-                                             double cohesion, double hardening, double anphi, double anpsi,
-                                             double st, double a1, double a2) {
+                                             double cohesion, double hardening, double anphi, double sq_anphi,
+                                             double aP, double anpsi, double st, double a1, double a2) {
     double alam, dep1, dep2, dep3, depm;
-    double fs = sp[0] - sp[2] * anphi + 2 * cohesion * sqrt(anphi);
+    double fs = sp[0] - sp[2] * anphi + 2 * cohesion * sq_anphi;
     double ft = sp[2] - st;
     if (!(fs < 0.0f || ft > 0.0f)) return 0;
-    double aP = sqrt(1.0f + anphi * anphi) + anphi;
-    double sP = st * anphi - 2 * cohesion * sqrt(anphi);
+    double sP = st * anphi - 2 * cohesion * sq_anphi;
     double h = sp[2] - st + aP * (sp[0] - sP);
     if (h < 0.0f) {
-        alam = dv(fs, a1 - a2 * anpsi + a1 * anphi * anpsi - a2 * anphi + 2.0 * sqrt(anphi) * hardening);
+        alam = dv(fs, a1 - a2 * anpsi + a1 * anphi * anpsi - a2 * anphi + 2.0 * sq_anphi * hardening);
         sp[0] -= alam * (a1 - a2 * anpsi);
         sp[1] -= alam * a2 * (1.0f - anpsi);
         sp[2] -= alam * (a2 - a1 * anpsi);

@@ -697,7 +697,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
     for (int a = 0; a < 6; a++) pst[a] = in.pst[a];
     if (PLUGIN == SNAC_RHEOLOGY_PLASTIC || is_vp(PLUGIN)) {
         double frictionAngle = fa, dilationAngle = da, cohesion = co, hardening = hd;
-        double stc, anphi, anpsi, sq_anphi;
+        double stc, anphi, anpsi, sq_anphi, aP;
         if (M.fric_const && M.dil_const && M.fric0 > 0.0 && __all_sync(FULL, matched)) {
             // the usual table: every tet of the warp found its segment, angles
             // constant, their sines and tangents evaluated on the host
@@ -707,6 +707,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
             anphi = M.anphi0;
             anpsi = M.anpsi0;
             sq_anphi = M.sq_anphi0;
+            aP = M.ap0;
         } else {
             // The reference keeps the table values (and the tension cutoff) in
             // variables that outlive the tet loop: a tet whose lookup matched no
@@ -749,6 +750,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
             anphi = fconst ? M.anphi0 : dv(1.0f + sphi, 1.0f - sphi);
             anpsi = (M.dil_const && dilationAngle == M.dil0) ? M.anpsi0 : dv(1.0f + spsi, 1.0f - spsi);
             sq_anphi = fconst ? M.sq_anphi0 : sqrt(anphi);
+            aP = fconst ? M.ap0 : sqrt(1.0f + anphi * anphi) + anphi;
         }
         if (PLUGIN == SNAC_VP_DP && !M.yield_mc) {
             // viscoplastic/Constitutive.c:372-518 (the principal stresses the
@@ -770,7 +772,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
                 stash_faces(g, r, row, areas, s.lane);
                 if (may_yield) {
                     principal_stresses(st, sp, cn);
-                    mc_return_map(sp, cn, st, eps_p, cohesion, hardening, anphi, anpsi, stc, a1, a2);
+                    mc_return_map(sp, cn, st, eps_p, cohesion, hardening, anphi, sq_anphi, aP, anpsi, stc, a1, a2);
                 }
                 unstash_faces(g, r, row, areas, s.lane);
             }
@@ -1928,6 +1930,8 @@ __global__ void k_selftest_division(long long n, unsigned long long seed, unsign
         if (((d >> 4) & 15) == 0) y = __longlong_as_double((long long)((b & 0x800fffffffffffffull) | ((d >> 20) % 2048) << 52));
         local += !same_bits(dv(x, y), x / y);
         local += !same_bits(dvz(x, y, recip(y)), x / y);
+        const double y1 = __longlong_as_double((long long)((a & 0x000fffffffffffffull) | ((unsigned long long)(1023 + (int)((c >> 12) % 64)) << 52)));
+        if (__double2loint(y1) != -1) local += !same_bits(recip_mid(y1), 1.0 / y1);
         // the joint root and reciprocal of tet_geometry_tame over its range, but
         // for the roots its caller turns away
         const double q = __longlong_as_double((long long)((b & 0x000fffffffffffffull) | ((unsigned long long)(1023 + (int)((c >> 8) % 1283) - 714) << 52)));
