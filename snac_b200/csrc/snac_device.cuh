@@ -357,31 +357,32 @@ __device__ __forceinline__ void tet_geometry(const V3 c[4], TetGeom& g) {
 }
 
 // ---- the same geometry for tame coordinates ------------------------------------------
-// A coordinate is tame when it is 0 or its magnitude lies in [2^-100, 2^140)
+// A coordinate is tame when it is 0 or its magnitude lies in [2^-100, 2^100)
 // (a length in metres always does, short of an exact 0 that a wave front has
 // just begun to move).  Then nothing in a tet's geometry needs a range test
 // of its own:
-//   an edge component (a difference) is 0 or in [2^-152, 2^141]: both
+//   an edge component (a difference) is 0 or in [2^-152, 2^101]: both
 //     coordinates are multiples of 2^-152;
-//   a product of two is 0 or in [2^-304, 2^282], a multiple of 2^-356 or
+//   a product of two is 0 or in [2^-304, 2^202], a multiple of 2^-356 or
 //     coarser after rounding, so a cross-product component is 0 or in
-//     [2^-357, 2^283];
-//   its square is 0 or in [2^-714, 2^566], a face's sum q of three in [2^-714, 2^568]
-//     unless all are 0, its root s in [2^-357, 2^284];
-//   the volume determinant is 0 or in [2^-562, 2^428].
+//     [2^-357, 2^203];
+//   its square is 0 or in [2^-714, 2^406], a face's sum q of three in [2^-714, 2^408]
+//     unless all are 0, its root s in [2^-357, 2^204];
+//   the volume determinant is 0 or in [2^-562, 2^308].
 // So the quotients by 6 and by s lie inside the windows of dvk and dvz, and the root
 // and RN(1/s) come from one reciprocal-root seed.  A face with q = 0, a
 // volume outside [2^-450, 2^451) and a root whose low word is all ones (which
 // covers the one significand whose reciprocal the last step below may round wrongly) turn
-// `ok` off; the caller then takes the general form.
-constexpr int TAME_LO = -100, TAME_HI = 139;
+// `ok` off; the caller then takes the general form.  Velocities are tame
+// below 2^240.
+constexpr int TAME_LO = -100, TAME_HI = 99, TAME_V = 240;
 __device__ __forceinline__ bool tame_coordinate(double x) { return zero_or_within<TAME_LO, TAME_HI>(x); }
-// |x| < 2^140 (false for infinities and NaN)
+// |x| < 2^TAME_V (false for infinities and NaN)
 __device__ __forceinline__ bool tame_size(double x) {
-    return ((unsigned)__double2hiint(x) & 0x7fffffffu) < ((unsigned)(1023 + TAME_HI + 1) << 20);
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) < ((unsigned)(1023 + TAME_V) << 20);
 }
 
-// s = RN(sqrt(q)) and z = RN(1/s) for q in [2^-714, 2^568]: Newton's coupled
+// s = RN(sqrt(q)) and z = RN(1/s) for q in [2^-714, 2^408]: Newton's coupled
 // iteration for sqrt(q) and 1/(2 sqrt(q)) from the hardware's approximate
 // reciprocal root (its error e goes to about 3/2 e^2 per pass: two passes
 // from 2^-20 reach rounding level), then Markstein's final steps, one FMA
@@ -464,8 +465,8 @@ __device__ __forceinline__ double shear_sum(const V3 v[4], const TetGeom& g, int
 
 // StrainRate.c:65-184, before the mixed-discretisation correction;
 // sr = (xx, yy, zz, xy, xz, yz)
-// tame: the tet's coordinates are tame, its velocities below 2^140 and its
-// volume in [2^-450, 2^451).  Then every sum is below 2^428, so the
+// tame: the tet's coordinates and velocities are tame and its volume in
+// [2^-450, 2^451).  Then every sum is below 2^448, so the
 // quotient by 3 needs no range test (for the divisor 3 the correction step is
 // exact for every finite x: the remainder is a multiple of the smallest
 // subnormal, and x / 3 never lies halfway between two doubles), and the

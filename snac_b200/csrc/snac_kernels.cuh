@@ -1697,10 +1697,31 @@ __device__ __forceinline__ void sync_one(const Config& cfg, DevScalars* sc, doub
 // The minimum length scale of the new coordinates and Sync in one launch:
 // the last block to finish (counted in DevScalars, reset by that block) runs
 // Sync on the completed reductions.
-constexpr int MINLS_THREADS = 128;  // one thread per hex
+// PER_TET: a thread per tet instead of a thread per hex.  A hex's ten tets share
+// their corner loads and edge differences in one thread, which is the better
+// form once the GPU is full (131 k hexes: 21 against 42 us); a small mesh's one
+// wave is done sooner with a tenth of the work per thread.
+constexpr int MINLS_THREADS = 128;
+static_assert(MINLS_THREADS == ELEM_WARPS * 32, "both forms have blocks of one size");
+template <bool PER_TET>
 __global__ void __launch_bounds__(MINLS_THREADS) k_min_length_scale_sync(Mesh m, Fields F, Config cfg,
                                                                          double wave_speed) {
-    double ls = hex_min_length_scale(m, F, blockIdx.x);
+    double ls;
+    if (PER_TET) {
+        __shared__ __align__(16) TripleCoords tri[ELEM_WARPS];
+        TripleCoords& z = tri[threadIdx.x >> 5];
+        fetch_triple<0>(m, F, blockIdx.x, z);
+        const TetLane L = tet_lane();
+        const TetSlot s = tet_slot_of(m, L, blockIdx.x);
+        cp_async_wait_all();
+        __syncwarp();
+        TetGeom g;
+        triple_geometry<false>(z, L, g);
+        ls = tet_length_scale(g);
+        if (s.active && g.V == 0.0) report(F.sc, SNAC_GPU_EVOLUME, s.e);
+    } else {
+        ls = hex_min_length_scale(m, F, blockIdx.x);
+    }
     for (int o = 16; o > 0; o >>= 1) ls = fmin(ls, __shfl_xor_sync(FULL, ls, o));
     // the block's minimum in one atomic (fewer atomics on the one address),
     // fenced so that it is visible device-wide before the block is counted

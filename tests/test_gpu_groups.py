@@ -40,7 +40,7 @@ def test_edges_of_groups_and_node_blocks(shape, kind):
     check(MAKE[kind](*shape))
 
 
-# lengths around 1e45 and 1e-35 m: outside [2^-100, 2^140), every triple takes the
+# lengths around 1e45 and 1e-35 m: outside [2^-100, 2^100), every triple takes the
 # general geometry; 1e-33 m on one node: that node's triples do, the others not
 @pytest.mark.parametrize("scale", [1.0e40, 1.0e-40])
 def test_untame_coordinates(scale):
