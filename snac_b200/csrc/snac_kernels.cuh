@@ -1994,6 +1994,56 @@ __global__ void k_unpack_nodes(double4* __restrict__ dst, const double* __restri
     }
 }
 
+// ---- arrays between the device and page-locked host memory that the device maps ---------
+// A few dozen copies of a state's pieces cost several microseconds each,
+// whatever their size; a kernel that reads or writes the host's arrays itself
+// costs one launch.  Rows: consecutive doubles of the host array; what: 0 the
+// same doubles on the device, 1 the x, y, z of a double4 per three, 2 the w of a double4 per one.
+struct HostRows {
+    double* host;
+    double* dev;
+    long long n;   // doubles
+    int what;
+};
+struct HostJob {
+    static constexpr int MAX = 10;
+    HostRows rows[MAX];
+    long long first[MAX + 1];  // first unit (two doubles) of each piece
+    int count;
+};
+__device__ __forceinline__ double* dev_double(const HostRows& r, long long i) {
+    return r.what == 0 ? r.dev + i : r.what == 1 ? r.dev + i / 3 * 4 + i % 3 : r.dev + i * 4 + 3;
+}
+template <bool TO_HOST>
+__global__ void __launch_bounds__(256) k_host_rows(HostJob J) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < J.first[J.count]; u += stride) {
+        int a = 0;
+        while (u >= J.first[a + 1]) a++;
+        // pairs that start on 16-byte boundaries of the host array: where it
+        // starts between two, its first unit is a single double
+        const HostRows& r = J.rows[a];
+        const int odd = (int)((unsigned long long)r.host >> 3) & 1;
+        const long long i = (u - J.first[a]) * 2 - odd;
+        if (i >= 0 && i + 1 < r.n) {
+            double2* const h = reinterpret_cast<double2*>(r.host + i);
+            if (TO_HOST) {
+                *h = make_double2(*dev_double(r, i), *dev_double(r, i + 1));
+            } else {
+                const double2 v = *h;
+                *dev_double(r, i) = v.x;
+                *dev_double(r, i + 1) = v.y;
+            }
+        } else {
+            const long long x = i < 0 ? 0 : i;
+            if (x < r.n) {
+                if (TO_HOST) r.host[x] = *dev_double(r, x);
+                else *dev_double(r, x) = r.host[x];
+            }
+        }
+    }
+}
+
 // The node state of nodes [0, nn) between the host's rows (3 doubles of
 // coordinates, 3 of velocity, 1 of temperature per node) and the device's
 // double4 rows (pos: x, y, z, T; vel: vx, vy, vz and the previous T, which
