@@ -1511,7 +1511,8 @@ static int record_host_step(snac_gpu* h, const snac_state_view* in, const snac_s
         if (in->stress) CK(cudaMemcpyAsync(h->stress + a * 6, in->stress + a * 6, n * 6 * D, cudaMemcpyHostToDevice, q->in));
         if (in->plastic_strain && h->eps_p)
             CK(cudaMemcpyAsync(h->eps_p + a, in->plastic_strain + a, n * D, cudaMemcpyHostToDevice, q->in));
-        if (in->viscosity && h->visc)
+        // the visco-plastic hook writes every tet's viscosity in this step and reads none
+        if (in->viscosity && h->visc && h->constitutive == SNAC_RHEOLOGY_MAXWELL)
             CK(cudaMemcpyAsync(h->visc + a, in->viscosity + a, n * D, cudaMemcpyHostToDevice, q->in));
         if (give_pst && h->pst)
             CK(cudaMemcpyAsync(h->pst + a * 6, in->plastic_strain_tensor + a * 6, n * 6 * D, cudaMemcpyHostToDevice, q->in));
@@ -1664,10 +1665,13 @@ int snac_gpu_step_host(snac_gpu* h, const snac_state_view* in, const snac_state_
     memcpy(&vi, in, vbytes);
     memcpy(&vo, out, vbytes);
     // default: one slab per 6 MiB of stresses (the bulk of the transfers),
-    // 1 to 16 slabs; smaller slabs cost more in per-slab latency than they
-    // save in pipeline fill
+    // up to 16 slabs; smaller slabs cost more in per-slab latency than they
+    // save in pipeline fill, but below six slabs the fill weighs more: one per 3 MiB there
+    // (45x21x37 visco-plastic: 3 slabs 1.03 ms, 6 slabs 0.95, 8 slabs 0.98)
     const long long stress_bytes = h->mesh.ne * NT * 6 * (long long)sizeof(double);
-    const int S = chunks ? chunks : (int)std::max(1LL, std::min(16LL, (stress_bytes + (3LL << 20)) / (6LL << 20)));
+    auto slabs_of = [&](long long unit) { return (stress_bytes + unit / 2) / unit; };
+    const int S = chunks ? chunks
+                         : (int)std::max({1LL, std::min(6LL, slabs_of(3LL << 20)), std::min(16LL, slabs_of(6LL << 20))});
     {
         // every return below waits for this call's copies first: the caller
         // may release its host buffers once the call has returned
