@@ -688,7 +688,7 @@ bool device_maps(const void* p, size_t bytes) {
             f = nullptr;
         return reinterpret_cast<Get>(f);
     }();
-    if (!get || !p) return false;
+    if (!get || !p || (uintptr_t)p % sizeof(double)) return false;  // the kernel stores whole doubles
     const CUdeviceptr c = (CUdeviceptr)(uintptr_t)p;
     CUdeviceptr dev = 0, start = 0;
     unsigned type = 0;
@@ -710,12 +710,11 @@ struct HostRowsJob {
         J.count++;
     }
 };
-template <bool TO_HOST>
 int host_rows(snac_gpu* h, const HostRowsJob& j, cudaStream_t st) {
     if (j.J.count == 0) return 0;
     const long long units = j.J.first[j.J.count];
     const unsigned blocks = (unsigned)std::min<long long>((units + 255) / 256, 8LL * h->n_sm);
-    k_host_rows<TO_HOST><<<blocks, 256, 0, st>>>(j.J);
+    k_host_rows<<<blocks, 256, 0, st>>>(j.J);
     h->launches++;
     return launch_check_named(h, "k_host_rows");
 }
@@ -1457,7 +1456,7 @@ int snac_gpu_download(snac_gpu* h, const snac_state_view* v) {
         else
             CK(cudaMemcpyAsync(p.host, p.dev, p.n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     }
-    if ((rc = host_rows<true>(h, job, h->stream))) return rc;
+    if ((rc = host_rows(h, job, h->stream))) return rc;
     CK(cudaStreamSynchronize(h->stream));
     if (v->plastic_strain && !h->eps_p) memset(v->plastic_strain, 0, nq * sizeof(double));
     if (v->viscosity && !h->visc) memset(v->viscosity, 0, nq * sizeof(double));
@@ -1509,23 +1508,44 @@ static int record_host_step(snac_gpu* h, const snac_state_view* in, const snac_s
         if (e1 <= e0) return 0;
         const long long a = e0 * NT, n = (e1 - e0) * NT;
         if (in->stress) CK(cudaMemcpyAsync(h->stress + a * 6, in->stress + a * 6, n * 6 * D, cudaMemcpyHostToDevice, q->in));
+        if (give_pst && h->pst)
+            CK(cudaMemcpyAsync(h->pst + a * 6, in->plastic_strain_tensor + a * 6, n * 6 * D, cudaMemcpyHostToDevice, q->in));
+        return 0;
+    };
+    // The arrays of one value per tet go in copies of several slabs: a copy
+    // costs the link about 5 us besides its bytes, and these are a sixth of
+    // the stresses.  Up with the first two slabs, then four at a time; back
+    // two at a time, as the last slabs' follow every kernel.  Plastic
+    // 80x40x70 (16 slabs) 3.9-4.2 ms with a copy per slab, 3.8 so, 3.98 with
+    // two up and one back, 3.9 with all at once; 60x30x60 2.13, 2.05, 2.10, 2.09.
+    constexpr int SCALARS_IN = 4, SCALARS_OUT = 2;
+    auto scalars_in = [&](int c) -> int {
+        if (!(c == 0 || (c >= 2 && (c - 2) % SCALARS_IN == 0))) return 0;
+        const int upto = std::min(S, c == 0 ? 2 : c + SCALARS_IN);
+        const long long a = E[c] * NT, n = (E[upto] - E[c]) * NT;
+        if (n <= 0) return 0;
         if (in->plastic_strain && h->eps_p)
             CK(cudaMemcpyAsync(h->eps_p + a, in->plastic_strain + a, n * D, cudaMemcpyHostToDevice, q->in));
         // the visco-plastic hook writes every tet's viscosity in this step and reads none
         if (in->viscosity && h->visc && h->constitutive == SNAC_RHEOLOGY_MAXWELL)
             CK(cudaMemcpyAsync(h->visc + a, in->viscosity + a, n * D, cudaMemcpyHostToDevice, q->in));
-        if (give_pst && h->pst)
-            CK(cudaMemcpyAsync(h->pst + a * 6, in->plastic_strain_tensor + a * 6, n * 6 * D, cudaMemcpyHostToDevice, q->in));
+        return 0;
+    };
+    auto scalars_out = [&](int c) -> int {
+        if (c != S - 1 && (c + 1) % SCALARS_OUT) return 0;
+        const int from = c / SCALARS_OUT * SCALARS_OUT;
+        const long long a = E[from] * NT, n = (E[c + 1] - E[from]) * NT;
+        if (n <= 0) return 0;
+        if (out->plastic_strain && h->eps_p)
+            CK(cudaMemcpyAsync(out->plastic_strain + a, h->eps_p + a, n * D, cudaMemcpyDeviceToHost, q->out));
+        if (out->viscosity && h->visc)
+            CK(cudaMemcpyAsync(out->viscosity + a, h->visc + a, n * D, cudaMemcpyDeviceToHost, q->out));
         return 0;
     };
     auto elems_out = [&](long long e0, long long e1) -> int {
         if (e1 <= e0) return 0;
         const long long a = e0 * NT, n = (e1 - e0) * NT;
         if (out->stress) CK(cudaMemcpyAsync(out->stress + a * 6, h->stress + a * 6, n * 6 * D, cudaMemcpyDeviceToHost, q->out));
-        if (out->plastic_strain && h->eps_p)
-            CK(cudaMemcpyAsync(out->plastic_strain + a, h->eps_p + a, n * D, cudaMemcpyDeviceToHost, q->out));
-        if (out->viscosity && h->visc)
-            CK(cudaMemcpyAsync(out->viscosity + a, h->visc + a, n * D, cudaMemcpyDeviceToHost, q->out));
         if (want_pst && h->pst)
             CK(cudaMemcpyAsync(out->plastic_strain_tensor + a * 6, h->pst + a * 6, n * 6 * D, cudaMemcpyDeviceToHost, q->out));
         return 0;
@@ -1568,6 +1588,7 @@ static int record_host_step(snac_gpu* h, const snac_state_view* in, const snac_s
             if ((rc = nodes_up(n_head, nn))) return rc;
             CK(cudaEventRecord(q->nodes_rest, q->in));
         }
+        if ((rc = scalars_in(c))) return rc;
         if ((rc = elems_in(E[c], E[c + 1]))) return rc;
         CK(cudaEventRecord(q->ev_in[c], q->in));
     }
@@ -1598,6 +1619,7 @@ static int record_host_step(snac_gpu* h, const snac_state_view* in, const snac_s
             continue;
         }
         if (o.kind == SlabOp::HEXES_BACK) {
+            if ((rc = scalars_out(o.slab))) return rc;
             if ((rc = elems_out(E[o.slab], E[o.slab + 1]))) return rc;
             continue;
         }

@@ -202,23 +202,6 @@ __device__ __forceinline__ double hex_total(const double (&h)[3 * 12], int base)
     return s;
 }
 
-// a tet's six stress components as three 16-byte accesses (the [nq][6]
-// rows start on 48-byte boundaries)
-__device__ __forceinline__ void load_stress(const Fields& F, long long q, double st[6]) {
-    const double2* p = reinterpret_cast<const double2*>(F.stress + q * 6);
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const double2 v = p[a];
-        st[2 * a] = v.x;
-        st[2 * a + 1] = v.y;
-    }
-}
-__device__ __forceinline__ void store_stress(const Fields& F, long long q, const double st[6]) {
-    double2* p = reinterpret_cast<double2*>(F.stress + q * 6);
-#pragma unroll
-    for (int a = 0; a < 3; a++) p[a] = make_double2(st[2 * a], st[2 * a + 1]);
-}
-
 struct TetSlot {
     int lane, base, t;
     long long e, q;
@@ -1996,8 +1979,8 @@ __global__ void k_unpack_nodes(double4* __restrict__ dst, const double* __restri
 
 // ---- arrays between the device and page-locked host memory that the device maps ---------
 // A few dozen copies of a state's pieces cost several microseconds each,
-// whatever their size; a kernel that reads or writes the host's arrays itself
-// costs one launch.  Rows: consecutive doubles of the host array; what: 0 the
+// whatever their size; a kernel that writes the host's arrays itself costs
+// one launch.  Rows: consecutive doubles of the host array; what: 0 the
 // same doubles on the device, 1 the x, y, z of a double4 per three, 2 the w of a double4 per one.
 struct HostRows {
     double* host;
@@ -2014,7 +1997,6 @@ struct HostJob {
 __device__ __forceinline__ double* dev_double(const HostRows& r, long long i) {
     return r.what == 0 ? r.dev + i : r.what == 1 ? r.dev + i / 3 * 4 + i % 3 : r.dev + i * 4 + 3;
 }
-template <bool TO_HOST>
 __global__ void __launch_bounds__(256) k_host_rows(HostJob J) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < J.first[J.count]; u += stride) {
@@ -2026,20 +2008,10 @@ __global__ void __launch_bounds__(256) k_host_rows(HostJob J) {
         const int odd = (int)((unsigned long long)r.host >> 3) & 1;
         const long long i = (u - J.first[a]) * 2 - odd;
         if (i >= 0 && i + 1 < r.n) {
-            double2* const h = reinterpret_cast<double2*>(r.host + i);
-            if (TO_HOST) {
-                *h = make_double2(*dev_double(r, i), *dev_double(r, i + 1));
-            } else {
-                const double2 v = *h;
-                *dev_double(r, i) = v.x;
-                *dev_double(r, i + 1) = v.y;
-            }
+            *reinterpret_cast<double2*>(r.host + i) = make_double2(*dev_double(r, i), *dev_double(r, i + 1));
         } else {
             const long long x = i < 0 ? 0 : i;
-            if (x < r.n) {
-                if (TO_HOST) r.host[x] = *dev_double(r, x);
-                else *dev_double(r, x) = r.host[x];
-            }
+            if (x < r.n) r.host[x] = *dev_double(r, x);
         }
     }
 }
