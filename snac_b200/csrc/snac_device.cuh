@@ -117,15 +117,19 @@ struct DevScalars {
     long long err_index;
     long long launches;
     double inertial_density0;        // (lambda + 2 mu) / c^2 of phase 0 at the current speed of sound c (dynamic dt)
-    unsigned blocks_done;            // blocks of k_min_length_scale_sync finished (0 between launches)
+    unsigned blocks_done;            // blocks of k_min_length_scale_sync or k_vmax_sync finished (0 between launches)
     unsigned pad;
+    int* told;                       // page-locked word of the host, nonzero once something has been reported
     // k_heat_flux_min_length_scale's per-block minima, spread over 32
     // addresses (+inf between steps)
     unsigned long long minls_slot[32];
 };
 
 __device__ __forceinline__ void report(DevScalars* sc, int code, long long index) {
-    if (atomicCAS(&sc->status, 0, code) == 0) sc->err_index = index;
+    if (atomicCAS(&sc->status, 0, code) == 0) {
+        sc->err_index = index;
+        *(volatile int*)sc->told = 1;  // the host sees it when the kernel has ended
+    }
 }
 
 #ifndef SNAC_MARKSTEIN_DIV

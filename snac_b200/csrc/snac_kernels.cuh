@@ -1799,8 +1799,16 @@ __device__ __forceinline__ void k_vmax_body(const Mesh& m, const Fields& F, int 
         atomicMax(&F.sc->vmax_bits, (unsigned long long)__double_as_longlong(vcand));
 }
 
-__global__ void __launch_bounds__(256) k_vmax(Mesh m, Fields F) {
+// With Sync in the same launch, run by the last block as in k_min_length_scale_sync
+// (both are latency alone: one launch less per hook-by-hook step).
+__global__ void __launch_bounds__(256) k_vmax_sync(Mesh m, Fields F, Config cfg, double wave_speed) {
     k_vmax_body(m, F, blockIdx.x);
+    __threadfence();  // each warp's maximum is visible device-wide before the block is counted
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(&F.sc->blocks_done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    sync_one(cfg, F.sc, wave_speed);
+    F.sc->blocks_done = 0u;
 }
 
 // ======================================================================================
