@@ -52,6 +52,33 @@ __device__ __forceinline__ void load_desc(ModelDesc& dst, const ModelDesc* __res
     for (int i = threadIdx.x; i < W; i += blockDim.x) d[i] = s[i];
 }
 
+// What a tile costs beyond the single-model kernel's block is the chain list
+// entry -> descriptor -> first loads, and the registers held across the body.
+// The tiles of one block: at(i) is tile i of the list, whose model's descriptor
+// is then in md for the whole block (the previous tile is done).  The list
+// entry of the block's next tile is fetched a tile ahead, and a descriptor
+// that is there already stays: consecutive tiles mostly are of one model.
+struct Tiles {
+    const ModelDesc* __restrict__ D;
+    const int2* __restrict__ list;
+    int n;
+    int2 next;
+    int model = -1;
+    __device__ __forceinline__ Tiles(const ModelDesc* __restrict__ D_, const int2* __restrict__ l, int n_)
+        : D(D_), list(l), n(n_), next(l[blockIdx.x]) {}  // (the grid is at most n blocks)
+    __device__ __forceinline__ int at(int i, ModelDesc& md) {
+        const int2 t = next;
+        if (i + (int)gridDim.x < n) next = list[i + gridDim.x];
+        __syncthreads();  // the previous tile is done with md and the staging
+        if (t.x != model) {
+            load_desc(md, D + t.x);
+            model = t.x;
+            __syncthreads();
+        }
+        return t.y;
+    }
+};
+
 // the element bodies for a tile's model: phase 0 from the descriptor (in
 // shared memory) when the model has one phase, else the model's phase table
 union TileSmem {
@@ -103,17 +130,15 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32, 4)
     kb_elements(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
     __shared__ ModelDesc md;
     __shared__ __align__(16) TileSmem S;
+    Tiles T(D, tiles, ntiles);
     for (int i = blockIdx.x; i < ntiles; i += gridDim.x) {
-        const int2 t = tiles[i];
-        __syncthreads();  // the previous tile is done with md
-        load_desc(md, D + t.x);
-        __syncthreads();
+        const int b = T.at(i, md);
         const bool temp = md.cfg.temperature != 0;
         switch (md.cfg.constitutive) {
-            case SNAC_RHEOLOGY_ELASTIC: elem_tile<OP, SNAC_RHEOLOGY_ELASTIC>(S, md, t.y, temp); break;
-            case SNAC_RHEOLOGY_PLASTIC: elem_tile<OP, SNAC_RHEOLOGY_PLASTIC>(S, md, t.y, temp); break;
-            case SNAC_RHEOLOGY_VISCOPLASTIC: elem_tile<OP, SNAC_RHEOLOGY_VISCOPLASTIC>(S, md, t.y, temp); break;
-            default: elem_tile<OP, SNAC_RHEOLOGY_MAXWELL>(S, md, t.y, temp); break;
+            case SNAC_RHEOLOGY_ELASTIC: elem_tile<OP, SNAC_RHEOLOGY_ELASTIC>(S, md, b, temp); break;
+            case SNAC_RHEOLOGY_PLASTIC: elem_tile<OP, SNAC_RHEOLOGY_PLASTIC>(S, md, b, temp); break;
+            case SNAC_RHEOLOGY_VISCOPLASTIC: elem_tile<OP, SNAC_RHEOLOGY_VISCOPLASTIC>(S, md, b, temp); break;
+            default: elem_tile<OP, SNAC_RHEOLOGY_MAXWELL>(S, md, b, temp); break;
         }
     }
 }
@@ -121,17 +146,22 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32, 4)
 // The same element-tile kernels specialised for one rheology class (plugin,
 // temperature on/off): the tile lists are grouped by class, and each class
 // present gets its own launch, without the run-time switch (fewer registers).
+// Resident blocks per SM asked of a class's kernel: as the single-model
+// kernels, but five of the heat flux (with both forms of the phase table and the
+// descriptor it spills twice as much at six; 24 models of up to 48x24x48: 460 us a
+// step with four for every class, 456 so).
+__host__ __device__ constexpr int tile_minb(int op, int plugin, bool temp) {
+    return op == BOP_HEAT_FLUX || (op == BOP_FUSED && temp) ? 5 : elem_minb(plugin);
+}
 template <int OP, int P, int TEMP>
-__global__ void __launch_bounds__(ELEM_WARPS * 32, 4)
+__global__ void __launch_bounds__(ELEM_WARPS * 32, tile_minb(OP, P, TEMP != 0))
     kb_elements_c(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
     __shared__ ModelDesc md;
     __shared__ __align__(16) TileSmem S;
+    Tiles T(D, tiles, ntiles);
     for (int i = blockIdx.x; i < ntiles; i += gridDim.x) {
-        const int2 t = tiles[i];
-        __syncthreads();
-        load_desc(md, D + t.x);
-        __syncthreads();
-        elem_tile<OP, P>(S, md, t.y, TEMP != 0);
+        const int b = T.at(i, md);
+        elem_tile<OP, P>(S, md, b, TEMP != 0);
     }
 }
 
@@ -155,30 +185,28 @@ __global__ void __launch_bounds__(256) kb_nodes(const ModelDesc* __restrict__ D,
     __shared__ GatherSmem S;
     if (OP != BOP_MINLS) gather_init(S);
     unsigned phase = 0;
+    Tiles T(D, tiles, ntiles);
     for (int i = blockIdx.x; i < ntiles; i += gridDim.x, phase ^= 1) {
-        const int2 t = tiles[i];
-        __syncthreads();
-        load_desc(md, D + t.x);
-        __syncthreads();
+        const int b = T.at(i, md);
         if (OP == BOP_LOOP_NODES) {
             const bool vo = md.cfg.vonly != 0;
             switch (md.cfg.dt_type) {
                 case SNAC_DT_CONSTANT:
-                    k_loop_nodes_body<SNAC_DT_CONSTANT, false>(S, md.m, md.F, md.cfg, t.y, 1, phase);
+                    k_loop_nodes_body<SNAC_DT_CONSTANT, false>(S, md.m, md.F, md.cfg, b, 1, phase);
                     break;
                 case SNAC_DT_DYNAMIC:
-                    if (vo) k_loop_nodes_body<SNAC_DT_DYNAMIC, true>(S, md.m, md.F, md.cfg, t.y, 1, phase);
-                    else k_loop_nodes_body<SNAC_DT_DYNAMIC, false>(S, md.m, md.F, md.cfg, t.y, 1, phase);
+                    if (vo) k_loop_nodes_body<SNAC_DT_DYNAMIC, true>(S, md.m, md.F, md.cfg, b, 1, phase);
+                    else k_loop_nodes_body<SNAC_DT_DYNAMIC, false>(S, md.m, md.F, md.cfg, b, 1, phase);
                     break;
                 default:
-                    if (vo) k_loop_nodes_body<SNAC_DT_WAVE, true>(S, md.m, md.F, md.cfg, t.y, 1, phase);
-                    else k_loop_nodes_body<SNAC_DT_WAVE, false>(S, md.m, md.F, md.cfg, t.y, 1, phase);
+                    if (vo) k_loop_nodes_body<SNAC_DT_WAVE, true>(S, md.m, md.F, md.cfg, b, 1, phase);
+                    else k_loop_nodes_body<SNAC_DT_WAVE, false>(S, md.m, md.F, md.cfg, b, 1, phase);
                     break;
             }
         } else if (OP == BOP_HEAT_NODES) {
-            k_heat_nodes_body(S, md.m, md.F, md.cfg, t.y, 1, phase);
+            k_heat_nodes_body(S, md.m, md.F, md.cfg, b, 1, phase);
         } else {
-            k_min_length_scale_body(md.m, md.F, t.y);
+            k_min_length_scale_body(md.m, md.F, b);
         }
     }
 }
