@@ -15,7 +15,7 @@
 //
 // Element kernels run one thread per tetrahedron: a warp holds three
 // elements in lanes 0-9, 10-19, 20-29 (lanes 30-31 idle).  Element sums
-// (volume, traces) are gathered lane by lane with shuffles and added in the
+// (volume, traces) go through shared memory and are added in the
 // reference's tet order, so they round like the reference's loops.  Node
 // kernels run one thread per node and gather the 8 adjacent hexes x 5 tets in
 // the reference's fixed order (Force.c:87-181): no atomics, bit-reproducible.
