@@ -862,6 +862,19 @@ int ensure_host_step(snac_gpu* h) {
     return 0;
 }
 
+// A page-locked word of its own for a handle.  The driver takes such memory from
+// the system a piece at a time and returns a piece with the last allocation in
+// it, each in 1 to 4 ms; while one allocation is held, another costs 6 us with
+// its release.  So four bytes stay held from the first handle of the process to its end.
+cudaError_t alloc_word(int** p) {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* held = nullptr;
+        if (cudaHostAlloc(&held, sizeof(int), cudaHostAllocMapped) != cudaSuccess) cudaGetLastError();  // then each handle pays
+    });
+    return cudaHostAlloc((void**)p, sizeof **p, cudaHostAllocMapped);
+}
+
 // hydroStaticIC/VariableConditions.c:43-152 on one rank: lithostatic
 // pressure integrated down each element column; densities are the phase
 // densities (tet densities are still zero at this point of the reference's IC).
@@ -1059,7 +1072,7 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
         CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     }
 
-    if (cudaHostAlloc((void**)&h->told, sizeof *h->told, cudaHostAllocMapped) != cudaSuccess)
+    if (alloc_word(&h->told) != cudaSuccess)
         return set_err(h, SNAC_GPU_ENOMEM, -1, "cudaHostAlloc(%zu bytes)", sizeof *h->told);
     *h->told = 0;
     const long long ne = m.ne, nn = m.nn, nq = ne * NT;
