@@ -681,9 +681,12 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
     if (PLUGIN == SNAC_RHEOLOGY_PLASTIC || is_vp(PLUGIN)) {
         double frictionAngle = fa, dilationAngle = da, cohesion = co, hardening = hd;
         double stc, anphi, anpsi, sq_anphi, aP;
-        if (M.fric_const && M.dil_const && M.fric0 > 0.0 && __all_sync(FULL, matched)) {
-            // the usual table: every tet of the warp found its segment, angles
-            // constant, their sines and tangents evaluated on the host
+        // the usual table: the tet found its segment, angles constant, their
+        // sines and tangents evaluated on the host.  The hexes of a warp may
+        // be of different phases, so the test itself is the tet's, and every
+        // lane takes the vote.
+        const bool usual = matched && M.fric_const && M.dil_const && M.fric0 > 0.0;
+        if (__all_sync(FULL, usual)) {
             stc = M.ten_off;
             const double tmp = dvz(cohesion, M.tan_fric0, M.ztan_fric0);
             if (tmp < stc) stc = tmp;
@@ -735,31 +738,30 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
             sq_anphi = fconst ? M.sq_anphi0 : sqrt(anphi);
             aP = fconst ? M.ap0 : sqrt(1.0f + anphi * anphi) + anphi;
         }
-        if (PLUGIN == SNAC_VP_DP && !M.yield_mc) {
-            // viscoplastic/Constitutive.c:372-518 (the principal stresses the
-            // reference computes first are not used by this branch)
-            if (s.active)
-                dp_return_map(st, dp_sd, dp_S0, e, dp_vic1, dp_vic2, M.mu, dp_bulkm, tan_fric(M, frictionAngle),
-                              tan_dil(M, dilationAngle), cohesion, stc, M.dp_tol, M.dp_maxit, pst, eps_p);
-        } else {
-            const double a1 = M.lambda + 2.0f * M.mu;
-            const double a2 = M.lambda;
-            // The reference always computes the principal stresses; they only
-            // matter when the tet yields.  A tet that provably stays inside the
-            // yield surface keeps its trial stress without the eigen-solve.
-            const bool may_yield = !surely_elastic(st, cohesion, anphi, sq_anphi, stc);
-            if (__any_sync(FULL, may_yield)) {
-                __syncwarp();  // every lane has read its corners
-                int row[4];
-                rows_of(row);
-                stash_faces(g, r, row, areas, s.lane);
-                if (may_yield) {
-                    principal_stresses(st, sp, cn);
-                    mc_return_map(sp, cn, st, eps_p, cohesion, hardening, anphi, sq_anphi, aP, anpsi, stc, a1, a2);
-                }
-                unstash_faces(g, r, row, areas, s.lane);
+        // a Drucker-Prager tet takes a return map of its own (the principal
+        // stresses the reference computes first are not used by it); its
+        // warp may hold Mohr-Coulomb tets, so it goes through their votes too
+        const bool dp = PLUGIN == SNAC_VP_DP && !M.yield_mc;
+        const double a1 = M.lambda + 2.0f * M.mu;
+        const double a2 = M.lambda;
+        // The reference always computes the principal stresses; they only
+        // matter when the tet yields.  A tet that provably stays inside the
+        // yield surface keeps its trial stress without the eigen-solve.
+        const bool may_yield = !dp && !surely_elastic(st, cohesion, anphi, sq_anphi, stc);
+        if (__any_sync(FULL, may_yield)) {
+            __syncwarp();  // every lane has read its corners
+            int row[4];
+            rows_of(row);
+            stash_faces(g, r, row, areas, s.lane);
+            if (may_yield) {
+                principal_stresses(st, sp, cn);
+                mc_return_map(sp, cn, st, eps_p, cohesion, hardening, anphi, sq_anphi, aP, anpsi, stc, a1, a2);
             }
+            unstash_faces(g, r, row, areas, s.lane);
         }
+        if (PLUGIN == SNAC_VP_DP && dp && s.active)  // viscoplastic/Constitutive.c:372-518
+            dp_return_map(st, dp_sd, dp_S0, e, dp_vic1, dp_vic2, M.mu, dp_bulkm, tan_fric(M, frictionAngle),
+                          tan_dil(M, dilationAngle), cohesion, stc, M.dp_tol, M.dp_maxit, pst, eps_p);
     }
 
     // trace averaging over the 10 tets, Stress.c:87-137
