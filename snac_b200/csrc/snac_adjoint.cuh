@@ -385,7 +385,6 @@ __device__ __forceinline__ void adj_tet_body(AdjSmem& sm, const Mesh& m, const F
         }
         R.clamped = past;
         if (s.active && seg < 0 && !past) report(F.sc, SNAC_GPU_ENOTSUP, s.e);  // the carried-over lookup is not differentiated
-        const bool angles_const = M.fric_const && M.dil_const;
         double fa = 0.0, co = 0.0, hd = 0.0, da = 0.0;
         if (seg >= 0) {
             const double dep = eps_p - M.plstrain[seg], dpl = M.plstrain[seg + 1] - M.plstrain[seg], zpl = M.zpl[seg];
@@ -394,7 +393,7 @@ __device__ __forceinline__ void adj_tet_body(AdjSmem& sm, const Mesh& m, const F
             co = c0 + hd * dep;
             fa = M.fric0;
             da = M.dil0;
-            if (!angles_const) {
+            if (!M.angles_const) {
                 const double f0 = M.fric[seg] * fsc;
                 double tg[2] = {M.fric[seg + 1] * fsc - f0, M.dil[seg + 1] - M.dil[seg]};
                 dvz_n(tg, dpl, zpl);

@@ -218,6 +218,11 @@ DevMaterial to_dev(const snac_material& s, bool fric_scaled, int dp_maxit, doubl
     }
     d.fric_const = fc;
     d.dil_const = dc;
+    d.angles_const = fc && dc;
+    for (int i = 0; i < s.nsegments; i++) {  // (a segment without width interpolates to NaN: 0 / 0)
+        const double width = s.plstrain[i + 1] - s.plstrain[i];
+        if (!(width > 0.0 && std::isfinite(width))) d.angles_const = 0;
+    }
     d.fric0 = s.friction_angle[0];
     d.sin_fric0 = sin(d.fric0 * degrad);
     d.tan_fric0 = tan(d.fric0 * degrad);

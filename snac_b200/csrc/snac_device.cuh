@@ -91,6 +91,7 @@ struct DevMaterial {
     double anphi0, anpsi0, sq_anphi0, ap0, ztan_fric0;  // ap0 = sqrt(1 + anphi0^2) + anphi0
     // host-evaluated transcendentals (valid when the *_const flag is set)
     int fric_const, dil_const;
+    int angles_const;  // both, and every segment of finite width > 0: a lookup gives the angles themselves
     double fric0, sin_fric0, tan_fric0;
     double dil0, sin_dil0, tan_dil0;
     // Drucker-Prager phase (yield_mc == 0, visco-plastic hook): maxiterations, constitutivetolerance

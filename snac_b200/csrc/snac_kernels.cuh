@@ -645,8 +645,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
         const double cs = in.coh;
         const double fsc = in.fric;
         // an angle that is the same at every point of the table keeps its
-        // value: 0 / dpl = 0 and angle + 0 * (eps_p - pl1) = angle
-        const bool angles_const = M.fric_const && M.dil_const;
+        // value: 0 / dpl = 0 and angle + 0 * (eps_p - pl1) = angle (dpl finite and not 0)
         for (int i = 0; i < M.nsegments; i++) {
             const double pl1 = M.plstrain[i], pl2 = M.plstrain[i + 1];
             if (eps_p >= pl1 && eps_p <= pl2) {
@@ -656,7 +655,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
                 co = c0 + hd * dep;
                 fa = M.fric0;
                 da = M.dil0;
-                if (!angles_const) {
+                if (!M.angles_const) {
                     const double f0 = M.fric[i] * fsc;
                     double tg[2] = {M.fric[i + 1] * fsc - f0, M.dil[i + 1] - M.dil[i]};
                     dvz_n(tg, dpl, zpl);
@@ -685,7 +684,7 @@ __device__ __forceinline__ void stress_update(const Mesh& m, const Fields& F, co
         // sines and tangents evaluated on the host.  The hexes of a warp may
         // be of different phases, so the test itself is the tet's, and every
         // lane takes the vote.
-        const bool usual = matched && M.fric_const && M.dil_const && M.fric0 > 0.0;
+        const bool usual = matched && M.angles_const && M.fric0 > 0.0;
         if (__all_sync(FULL, usual)) {
             stc = M.ten_off;
             const double tmp = dvz(cohesion, M.tan_fric0, M.ztan_fric0);

@@ -85,3 +85,24 @@ def test_batched_models_of_mixed_phases(split):
                 g.step(20)
                 for f in FIELDS:
                     assert np.array_equal(getattr(g.state(), f), getattr(m.state(), f)), f
+
+
+def test_softening_segment_without_width():
+    """A lookup in a segment of width 0 interpolates with 0 / 0: the angles become
+    NaN, also where they are the same at both ends, and the tension cutoff is
+    the one carried over (0 in an element's first tets), as in the oracle."""
+    cfg = VISCO(5, 3, 5)
+    cfg.materials = [phase(cfg, 30.0, 30.0)]
+    cfg.materials[0].update(nsegments=1, plstrain1=0.0, cohesion1=cfg.materials[0]["cohesion0"])
+    with SnacContext(cfg) as g:
+        c = Checker(cfg, "port")
+        g.time_step_zero()
+        c.time_step_zero()
+        g.step(20)
+        c.step(20)
+        sg, sc = g.state(), c.state()
+    assert np.count_nonzero(sc.plastic_strain) > 0
+    for f in FIELDS:
+        x, y = getattr(sg, f), getattr(sc, f)
+        assert np.all(np.isfinite(y)), f
+        assert np.max(np.abs(x - y)) <= 1e-6 * np.max(np.abs(y)), f
