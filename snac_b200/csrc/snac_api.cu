@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstddef>
@@ -76,6 +77,7 @@ struct snac_gpu {
     int has_density = 0;
     int n_phases = 0;
     double wave_speed = 0.0;
+    int device = 0;
     int n_sm = 148;
     cudaStream_t stream = nullptr;
     bool own_stream = true;  // false for the models of a batch, which share the batch's stream
@@ -278,6 +280,7 @@ unsigned elem_blocks(const Mesh& m) { return (unsigned)((m.ne + ELEM_PER_BLOCK -
 // stage.  As many stages as let every block of the grid be resident at once
 // (227 KB of shared memory per SM, of which a block takes 1 KB besides), else one:
 // a grid of more than one wave hides a pair's latency behind its other blocks.
+constexpr int GATHER_STAGES = 4;
 struct NodeLaunch {
     unsigned blocks;
     int stages;
@@ -287,15 +290,14 @@ NodeLaunch node_launch(const snac_gpu* h, unsigned blocks, int rows) {
     NodeLaunch l;
     l.blocks = blocks;
     const size_t stage = gather_stage_bytes(rows, NODE_THREADS);
-    for (l.stages = 4; l.stages > 1; l.stages /= 2)
+    for (l.stages = GATHER_STAGES; l.stages > 1; l.stages /= 2)
         if (blocks <= (227u << 10) / (l.stages * stage + 1024) * (unsigned)h->n_sm) break;
     l.smem = (size_t)l.stages * stage;
     return l;
 }
 unsigned node_blocks(const Mesh& m) { return (unsigned)((m.nn + NODE_THREADS - 1) / NODE_THREADS); }
-int force_rows(const snac_gpu* h) {
-    const bool cdt = h->cfg.dt_type == SNAC_DT_CONSTANT;
-    return force_chunk(cdt) + force_tail(cdt, h->cfg.vonly != 0);
+constexpr int force_rows(int dt_type, bool vonly) {
+    return force_chunk(dt_type == SNAC_DT_CONSTANT) + force_tail(dt_type == SNAC_DT_CONSTANT, vonly);
 }
 // The minimum length scale takes a thread per tet while its blocks (12 hexes)
 // fit one wave of the GPU (8 resident per SM), a thread per hex beyond.
@@ -303,11 +305,22 @@ int force_rows(const snac_gpu* h) {
 #define MINLS_TET 8
 #endif
 constexpr int MINLS_TET_BLOCKS_PER_SM = MINLS_TET;
-template <class K>
-cudaError_t allow_smem(K kernel, size_t bytes) {
-    return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
-                             : cudaSuccess;
+// Raises a kernel's limit of dynamic shared memory to `most`, the largest size
+// that any launch of it asks for.  The limit belongs to the kernel on a
+// device, not to a handle: were it set to what each launch needs, one thread
+// could lower it between another's call and launch.  So it takes one value only.
+template <auto KERNEL>
+cudaError_t allow_smem(int device, size_t most) {
+    static std::atomic<unsigned long long> done{0};  // devices 0 to 63
+    const unsigned long long bit = device < 64 ? 1ull << device : 0ull;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
 }
+// of a node gather: its most stages
+constexpr size_t most_stages(int rows) { return GATHER_STAGES * gather_stage_bytes(rows, NODE_THREADS); }
+static_assert(most_stages(CCHUNK) <= 227 * 1024, "the widest gather's stages fit an SM");
 
 // called right after each launch: checks it and, when profiling, records an
 // event behind it (the event before the first launch is recorded by the caller)
@@ -391,7 +404,7 @@ int op_fused_stress(snac_gpu* h) {
 int op_energy_nodes(snac_gpu* h, int count_step = 0) {
     if (!h->temperature) return 0;
     const NodeLaunch l = node_launch(h, node_blocks(h->mesh), HEAT_CHUNK + HEAT_TAIL);
-    CK(allow_smem(k_heat_nodes, l.smem));
+    CK(allow_smem<k_heat_nodes>(h->device, most_stages(HEAT_CHUNK + HEAT_TAIL)));
     k_heat_nodes<<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, fields(h), h->cfg, count_step, l.stages);
     h->launches++;
     if (count_step) h->time_step++;
@@ -417,8 +430,8 @@ int op_calc_stresses(snac_gpu* h) {
 
 template <int DT, bool VO>
 int launch_loop_nodes(snac_gpu* h, const Fields& F) {
-    const NodeLaunch l = node_launch(h, node_blocks(h->mesh), force_rows(h));
-    CK(allow_smem(k_loop_nodes<DT, VO>, l.smem));
+    const NodeLaunch l = node_launch(h, node_blocks(h->mesh), force_rows(DT, VO));
+    CK((allow_smem<k_loop_nodes<DT, VO>>(h->device, most_stages(force_rows(DT, VO)))));
     k_loop_nodes<DT, VO><<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, F, h->cfg, l.stages);
     return 0;
 }
@@ -788,8 +801,8 @@ int op_calc_stresses_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
 
 template <int DT, bool VO>
 int launch_loop_nodes_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
-    const NodeLaunch l = node_launch(h, (unsigned)(b1 - b0), force_rows(h));
-    CK(allow_smem(k_loop_nodes_slab<DT, VO>, l.smem));
+    const NodeLaunch l = node_launch(h, (unsigned)(b1 - b0), force_rows(DT, VO));
+    CK((allow_smem<k_loop_nodes_slab<DT, VO>>(h->device, most_stages(force_rows(DT, VO)))));
     k_loop_nodes_slab<DT, VO><<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, F, h->cfg, b0, l.stages);
     return 0;
 }
@@ -839,7 +852,7 @@ int op_heat_flux_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
 int op_heat_nodes_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     if (b1 <= b0) return 0;
     const NodeLaunch l = node_launch(h, (unsigned)(b1 - b0), HEAT_CHUNK + HEAT_TAIL);
-    CK(allow_smem(k_heat_nodes_slab, l.smem));
+    CK(allow_smem<k_heat_nodes_slab>(h->device, most_stages(HEAT_CHUNK + HEAT_TAIL)));
     k_heat_nodes_slab<<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, F, h->cfg, b0, l.stages);
     h->launches++;
     return launch_check_named(h, "k_heat_nodes_slab");
@@ -1066,7 +1079,7 @@ static int create_model(const snac_gpu_desc* d_in, snac_gpu** out, cudaStream_t 
     {
         int dev = 0, sms = 0;
         if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-            h->n_sm = sms;
+            h->device = dev, h->n_sm = sms;
     }
     c.pisos = d->pisos;  // replaced below when the hydrostatic IC runs here
     c.rzbo = d->rzbo;
@@ -1825,6 +1838,7 @@ struct snac_gpu_batch {
     std::vector<snac_gpu*> models;
     cudaStream_t stream = nullptr;
     int n = 0;
+    int device = 0;
     int n_sm = 148;
     ModelDesc* desc[2] = {nullptr, nullptr};  // [parity]
     int2* tiles = nullptr;
@@ -1971,7 +1985,7 @@ template <int OP>
 int blaunch_nodes(snac_gpu_batch* b, const ModelDesc* D, const snac_gpu_batch::List& L, int threads) {
     if (L.n == 0) return 0;
     const size_t smem = OP == BOP_MINLS ? 0 : node_stage_bytes(OP, threads);
-    BCK(allow_smem(kb_nodes<OP>, smem));
+    if (OP != BOP_MINLS) BCK(allow_smem<kb_nodes<OP>>(b->device, node_stage_bytes(OP, NODE_TILE_MAX)));
     kb_nodes<OP><<<tile_grid(b, L.n, b->tune.node_blocks_per_sm), threads, smem, b->stream>>>(D, b->tiles + L.off, L.n);
     return bcheck_launch(b, "kb_nodes");
 }
@@ -2146,6 +2160,7 @@ int snac_gpu_batch_create(const snac_gpu_desc* descs, int n_models, snac_gpu_bat
     *out = b;
     int dev = 0;
     BCK(cudaGetDevice(&dev));
+    b->device = dev;
     BCK(cudaDeviceGetAttribute(&b->n_sm, cudaDevAttrMultiProcessorCount, dev));
     BCK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     BCK(cudaEventCreate(&b->ev[0]));
@@ -2239,7 +2254,7 @@ int snac_gpu_batch_get_tuning(const snac_gpu_batch* b, snac_batch_tuning* out) {
 
 int snac_gpu_batch_set_tuning(snac_gpu_batch* b, const snac_batch_tuning* t) {
     if (!b || !t) return SNAC_GPU_EINVAL;
-    auto threads_ok = [](int x) { return x >= 32 && x <= 256 && x % 32 == 0; };
+    auto threads_ok = [](int x) { return x >= 32 && x <= NODE_TILE_MAX && x % 32 == 0; };
     if (!threads_ok(t->node_threads) || !threads_ok(t->minls_threads) || t->elem_blocks_per_sm < 0 ||
         t->elem_blocks_per_sm > 32 || t->node_blocks_per_sm < 0 || t->node_blocks_per_sm > 32 ||
         t->steps_per_graph < 1 || t->steps_per_graph > 256 || (t->order != 0 && t->order != 1) ||
@@ -2459,7 +2474,7 @@ int adjoint_supported(snac_gpu* h) {
 template <int P>
 int adj_tet_launch_p(snac_gpu* h, const Fields& F, const AdjState& S, const AdjBufs& B, int rotate, int first_rev,
                      double dt) {
-    CK(allow_smem(k_adj_tet<P>, sizeof(AdjSmem)));
+    CK(allow_smem<k_adj_tet<P>>(h->device, sizeof(AdjSmem)));
     k_adj_tet<P><<<elem_blocks(h->mesh), ELEM_WARPS * 32, sizeof(AdjSmem), h->stream>>>(h->mesh, F, h->cfg, S, B, rotate,
                                                                                        first_rev, dt);
     return 0;
@@ -2482,7 +2497,7 @@ int adj_tet_launch(snac_gpu* h, const AdjState& S, const AdjBufs& B, int rotate,
 int adj_nodes_launch(snac_gpu* h, const AdjState& cur, const AdjState& prev, const AdjBufs& B, int gather, int update,
                      double dt) {
     const NodeLaunch l = node_launch(h, node_blocks(h->mesh), CCHUNK);
-    CK(allow_smem(k_adj_nodes, l.smem));
+    CK(allow_smem<k_adj_nodes>(h->device, most_stages(CCHUNK)));
     k_adj_nodes<<<l.blocks, NODE_THREADS, l.smem, h->stream>>>(h->mesh, fields(h), cur, prev, B, gather, update, dt,
                                                               h->cfg.demf, l.stages);
     h->launches++;

@@ -179,8 +179,9 @@ __host__ __device__ constexpr int plugin_slot(int constitutive) {
 __host__ __device__ constexpr size_t node_stage_bytes(int op, int threads) {
     return gather_stage_bytes(op == BOP_HEAT_NODES ? HEAT_CHUNK + HEAT_TAIL : 50, threads);
 }
+constexpr int NODE_TILE_MAX = 256;  // nodes (threads) of the largest node tile
 template <int OP>
-__global__ void __launch_bounds__(256) kb_nodes(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
+__global__ void __launch_bounds__(NODE_TILE_MAX) kb_nodes(const ModelDesc* __restrict__ D, const int2* __restrict__ tiles, int ntiles) {
     __shared__ ModelDesc md;
     __shared__ GatherSmem S;
     if (OP != BOP_MINLS) gather_init(S);
