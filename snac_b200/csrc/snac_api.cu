@@ -2382,7 +2382,6 @@ constexpr size_t ADJ_KEEP = (size_t)512 << 20;
 int adj_ws_reserve(snac_gpu* h, size_t bytes) {
     if (h->adj_ws_bytes >= bytes) return 0;
     if (h->adj_ws) cudaFree(h->adj_ws);  // waits for whatever still uses it
-    h->alloc_bytes -= (long long)h->adj_ws_bytes;
     h->adj_ws = nullptr;
     h->adj_ws_bytes = 0;
     cudaError_t e = cudaMalloc(&h->adj_ws, bytes);
@@ -2391,13 +2390,12 @@ int adj_ws_reserve(snac_gpu* h, size_t bytes) {
         return set_err(h, SNAC_GPU_ENOMEM, -1, "adjoint workspace: cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
     }
     h->adj_ws_bytes = bytes;
-    h->alloc_bytes += (long long)bytes;
+    h->alloc_bytes += (long long)bytes;  // counts what was allocated: a release takes nothing back
     return 0;
 }
 void adj_ws_trim(snac_gpu* h) {
     if (h->adj_ws_bytes <= ADJ_KEEP) return;
     cudaFree(h->adj_ws);
-    h->alloc_bytes -= (long long)h->adj_ws_bytes;
     h->adj_ws = nullptr;
     h->adj_ws_bytes = 0;
 }

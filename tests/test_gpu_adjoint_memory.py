@@ -1,0 +1,41 @@
+"""Device memory of the adjoint: what snac_gpu_device_bytes says of its
+workspace."""
+import ctypes as C
+
+import pytest
+
+from snac_b200 import workloads as W
+from snac_b200.adjoint import adjoint, misfit, top_surface
+from snac_b200.context import SnacContext, load_library
+
+pytestmark = pytest.mark.gpu
+
+
+def device_bytes(ctx) -> int:
+    lib = load_library()
+    lib.snac_gpu_device_bytes.argtypes = [C.c_void_p, C.POINTER(C.c_longlong)]
+    lib.snac_gpu_device_bytes.restype = C.c_int
+    b = C.c_longlong(-1)
+    ctx._check(lib.snac_gpu_device_bytes(ctx.h, C.byref(b)))
+    return b.value
+
+
+def model():
+    g = SnacContext(W.c5_adjoint(32, 16, 32))
+    g.time_step_zero()
+    return g, top_surface(g.cfg, g.state())
+
+
+def test_device_bytes_never_decrease():
+    """A workspace of some 700 MB (60 states kept) is larger than what stays
+    allocated between calls; the count is of bytes allocated since creation."""
+    g, target = model()
+    with g:
+        last = device_bytes(g)
+        for call in (lambda: misfit(g, *target), lambda: adjoint(g, 12, *target),
+                     lambda: adjoint(g, 60, *target, checkpoint_every=1), lambda: misfit(g, *target),
+                     lambda: adjoint(g, 12, *target)):
+            call()
+            now = device_bytes(g)
+            assert now >= last
+            last = now
