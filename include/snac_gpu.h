@@ -385,7 +385,11 @@ int  snac_gpu_selftest_division(long long n, unsigned long long seed, long long*
  * temperature held fixed (thermal_conduct = 0); otherwise SNAC_GPU_ENOTSUP.
  * (The parameter gradients of the elastic and Maxwell hooks are zero: no
  * scale enters them; snac_gpu_adjoint_grads also returns the gradients with
- * respect to the initial state.) */
+ * respect to the initial state.)
+ * Device memory: a call (snac_gpu_misfit too) allocates one workspace, for
+ * the states it keeps and the adjoints.  It stays with the handle for the
+ * next call while all handles of the process keep 512 MiB at most, else it is
+ * released when the call ends; snac_gpu_destroy releases it. */
 typedef struct snac_adjoint_desc {
     int nsteps;
     int checkpoint_every;

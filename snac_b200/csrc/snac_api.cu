@@ -113,8 +113,9 @@ struct snac_gpu {
     double* topo_scratch = nullptr;  // [nnx * nnz] topography-diffusion scratch
     OutputState* out = nullptr;
     HostStep* hs = nullptr;  // snac_gpu_step_host's streams and staging
-    void* adj_ws = nullptr;  // the adjoint's workspace, kept for the next call (see ADJ_KEEP)
+    void* adj_ws = nullptr;  // the adjoint's workspace
     size_t adj_ws_bytes = 0;
+    bool adj_ws_kept = false;  // it stays for the next call (see ADJ_KEEP)
     // host mirror of the step bookkeeping
     int parity = 0;
     long long time_step = 0;
@@ -275,6 +276,8 @@ Fields fields_at(const snac_gpu* h, int parity) {
 Fields fields(const snac_gpu* h) { return fields_at(h, h->parity); }
 
 unsigned elem_blocks(const Mesh& m) { return (unsigned)((m.ne + ELEM_PER_BLOCK - 1) / ELEM_PER_BLOCK); }
+
+void adj_ws_release(snac_gpu* h);  // with the adjoint
 
 // The launch of a node gather over blocks of NODE_THREADS nodes; rows: of a
 // stage.  As many stages as let every block of the grid be resident at once
@@ -1320,9 +1323,10 @@ void snac_gpu_destroy(snac_gpu* h) {
     }
     void* bufs[] = {h->pos[0], h->pos[1], h->vel, h->force, h->stress, h->eps_p, h->pst, h->visc, h->density, h->vol,
                     h->hflux, h->tpre, h->fterm, h->bc, h->vbc_val, h->tbc_val, h->mat, h->mats, h->coh_scale, h->fric_scale,
-                    h->visc_scale, h->sc, h->stage, h->escal, h->residual_fr, h->topo_scratch, h->adj_ws};
+                    h->visc_scale, h->sc, h->stage, h->escal, h->residual_fr, h->topo_scratch};
     for (void* b : bufs)
         if (b) cudaFree(b);
+    adj_ws_release(h);
     if (h->told) cudaFreeHost(h->told);
     if (h->stream && h->own_stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -2375,15 +2379,23 @@ struct Carver {
         used += ((size_t)n * sizeof(T) + 255) & ~(size_t)255;
     }
 };
-// the handle keeps a workspace up to this size between calls; a larger one is
-// released when its call ends
+// A call's workspace stays with its handle for the next call while the handles of the process
+// keep this much in all; one that would exceed it is released when its call
+// ends.  32x16x32, 60 steps: 12.4 ms a call with it kept, 13.5 without;
+// 10x6x8, 24 steps: 2.5 and 3.2; a misfit 0.03 and 0.7.
 constexpr size_t ADJ_KEEP = (size_t)512 << 20;
+std::atomic<size_t> g_adj_kept{0};
 
-int adj_ws_reserve(snac_gpu* h, size_t bytes) {
-    if (h->adj_ws_bytes >= bytes) return 0;
+void adj_ws_release(snac_gpu* h) {
+    if (h->adj_ws_kept) g_adj_kept -= h->adj_ws_bytes;
     if (h->adj_ws) cudaFree(h->adj_ws);  // waits for whatever still uses it
     h->adj_ws = nullptr;
     h->adj_ws_bytes = 0;
+    h->adj_ws_kept = false;
+}
+int adj_ws_reserve(snac_gpu* h, size_t bytes) {
+    if (h->adj_ws_bytes >= bytes) return 0;
+    adj_ws_release(h);
     cudaError_t e = cudaMalloc(&h->adj_ws, bytes);
     if (e != cudaSuccess) {
         h->adj_ws = nullptr;
@@ -2393,11 +2405,16 @@ int adj_ws_reserve(snac_gpu* h, size_t bytes) {
     h->alloc_bytes += (long long)bytes;  // counts what was allocated: a release takes nothing back
     return 0;
 }
+// at the end of a call: keeps the workspace if the process may, releases it otherwise
 void adj_ws_trim(snac_gpu* h) {
-    if (h->adj_ws_bytes <= ADJ_KEEP) return;
-    cudaFree(h->adj_ws);
-    h->adj_ws = nullptr;
-    h->adj_ws_bytes = 0;
+    if (!h->adj_ws || h->adj_ws_kept) return;
+    size_t kept = g_adj_kept.load();
+    while (kept + h->adj_ws_bytes <= ADJ_KEEP)
+        if (g_adj_kept.compare_exchange_weak(kept, kept + h->adj_ws_bytes)) {
+            h->adj_ws_kept = true;
+            return;
+        }
+    adj_ws_release(h);
 }
 
 void snap_take(const snac_gpu* h, Carver& c, Snap& z) {

@@ -1,8 +1,9 @@
 """Device memory of the adjoint: what snac_gpu_device_bytes says of its
-workspace."""
+workspace, and how much stays allocated between calls."""
 import ctypes as C
 
 import pytest
+import torch
 
 from snac_b200 import workloads as W
 from snac_b200.adjoint import adjoint, misfit, top_surface
@@ -39,3 +40,25 @@ def test_device_bytes_never_decrease():
             now = device_bytes(g)
             assert now >= last
             last = now
+
+
+def test_handles_keep_a_bounded_workspace_together():
+    """Each handle's workspace is well over 100 MB; six handles keep at most 512 MiB
+    between their calls, and destroying them gives all of it back."""
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    models = [model() for _ in range(6)]
+    before = free()
+    for g, target in models:
+        adjoint(g, 12, *target)
+    # beside the workspaces a call leaves a few hundred KB of staging and graphs
+    slack = 16 << 20
+    assert before - free() <= (512 << 20) + slack * len(models)
+    first = models[0]
+    a, b = adjoint(first[0], 6, *first[1]), adjoint(models[-1][0], 6, *models[-1][1])
+    assert a.loss == b.loss  # one handle's workspace kept, the other's not
+    for g, _ in models:
+        g.close()
+    assert free() >= before
