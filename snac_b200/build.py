@@ -3,8 +3,12 @@
     python -m snac_b200.build          # rebuild if a source changed
     python -m snac_b200.build --force
 
-The library is one CUDA translation unit compiled with -fmad=false so that
-every kernel rounds like the reference's x86-64 build (see csrc/snac_device.cuh).
+The CUDA files are compiled side by side, one nvcc each, with -fmad=false so
+that every kernel rounds like the reference's x86-64 build (see
+csrc/snac_device.cuh).  Which kernels share a file decides what their calls
+cost in registers (csrc/snac_launch.cuh); no file is split among threads
+(-split-compile), whose grouping, and with it the code, differs from one
+build to the next.
 """
 from __future__ import annotations
 
@@ -13,6 +17,7 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -41,24 +46,29 @@ def stale() -> bool:
     return any(os.path.getmtime(s) > t for s in sources())
 
 
-# The count is fixed: it decides which kernels are register-allocated together
-# (noinline functions are shaped for the tightest of their callers), and 0 takes it from the
-# load of the building machine.  In one or two parts the batch's plastic kernel spills 240
-# bytes per thread and the fused plastic step 72; in four, eight or sixteen
-# neither does: 24 models of up to 48x24x48, 513 against 456 us a step.
-SPLIT = ["-split-compile=8"]
+def compile_commands(into: str, verbose: bool = False, defines=()):
+    """One nvcc command for each CUDA file, its object in the folder `into`."""
+    flags = [*ARCH, *["-D" + d for d in defines], "-lineinfo", "-O3", "-fmad=false", "-std=c++17",
+             "-Xcompiler", "-fPIC,-O2", "-I" + os.path.join(ROOT, "include")]
+    if verbose:
+        flags.insert(0, "-Xptxas=-v")
+    return [[nvcc(), *flags, "-c", "-o", os.path.join(into, os.path.basename(cu) + ".o"), cu]
+            for cu in sorted(glob.glob(os.path.join(CSRC, "*.cu")))]
 
 
 def build(force: bool = False, verbose: bool = False, defines=(), out: str = LIB) -> str:
     if not force and not stale() and out == LIB:
         return LIB
-    cmd = [nvcc(), *ARCH, *["-D" + d for d in defines], "-lineinfo", "-O3", *SPLIT, "-fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
-           "-shared", "-I" + os.path.join(ROOT, "include"), "-o", out + ".tmp",
-           os.path.join(CSRC, "snac_api.cu")]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-        print(" ".join(cmd))
-    subprocess.run(cmd, check=True)
+    with tempfile.TemporaryDirectory() as tmp:
+        commands = compile_commands(tmp, verbose, defines)
+        if verbose:
+            print("\n".join(" ".join(c) for c in commands), flush=True)
+        compilers = [subprocess.Popen(c) for c in commands]
+        failed = [c for c, p in zip(commands, compilers) if p.wait() != 0]
+        if failed:
+            raise subprocess.CalledProcessError(1, failed[0])
+        objects = [c[c.index("-o") + 1] for c in commands]
+        subprocess.run([nvcc(), *ARCH, "-shared", "-o", out + ".tmp", *objects], check=True)
     os.replace(out + ".tmp", out)
     return out
 

@@ -868,124 +868,4 @@ __global__ void __launch_bounds__(ELEM_WARPS * 32, SNAC_ADJ_MINB) k_adj_tet(Mesh
     adj_tet_body<PLUGIN>(*reinterpret_cast<AdjSmem*>(g_gather), m, F, cfg, S, B, rotate, first_rev, dt, blockIdx.x);
 }
 
-// Node adjoints: gather the corner adjoints of tet pass n (fixed order), then
-// the reverse of the node update of step n-1:
-//   x^n = x^{n-1} + dt v^n,  v^n_c = v^{n-1}_c + dt F_d,c / m  (free components)
-//   F_d = F (1 - demf sgn(v^{n-1}) sgn(F))
-// cur = S^n (its force holds F_d and m of step n-1), prev = S^{n-1} (velocities).
-__global__ void __launch_bounds__(NODE_THREADS) k_adj_nodes(Mesh m, Fields F, AdjState cur, AdjState prev, AdjBufs B,
-                                                           int gather, int update, double dt, double demf, int stages) {
-    __shared__ GatherSmem S;
-    const int n = blockIdx.x * NODE_THREADS + threadIdx.x;
-    const bool active = n < (int)m.nn;
-    double4 xb = make_double4(0.0, 0.0, 0.0, 0.0), vb = xb;
-    if (active) {
-        xb = B.xbar[n];
-        vb = B.vbar[n];
-    }
-    if (gather) {
-        gather_init(S);
-        int i = 0, j = 0, k = 0;
-        if (active) split3(n, m.nnx, m.nny, i, j, k);
-        const Gather<CCHUNK, 0> G{S, B.cbuf, CROWS, stages, gather_groups(NODE_THREADS) * CCHUNK * GROUP, 0};
-        const bool ok = G.run(m, blockIdx.x, active, i, j, k, [&](int ne, const double* r) {
-#pragma unroll
-            for (int idx = 0; idx < 5; idx++) {
-                const double* const o = r + pair_slot(ne, idx) * GROUP;
-                xb.x += o[0];
-                xb.y += o[ROW10];
-                xb.z += o[2 * ROW10];
-                vb.x += o[3 * ROW10];
-                vb.y += o[4 * ROW10];
-                vb.z += o[5 * ROW10];
-            }
-        });
-        if (!ok) report(F.sc, SNAC_GPU_ETIMEDOUT, n);
-    }
-    if (!active) return;
-    if (update) {
-        vb.x += dt * xb.x;
-        vb.y += dt * xb.y;
-        vb.z += dt * xb.z;
-        const double4 fd = cur.force[n];
-        const double4 vp = prev.vel[n];
-        const uchar4 bc = F.bc[n];
-        const double mass = fd.w;
-        double fb[3], mb = 0.0;
-        const double vbc[3] = {vb.x, vb.y, vb.z};
-        const double fdc[3] = {fd.x, fd.y, fd.z};
-        const double vpc[3] = {vp.x, vp.y, vp.z};
-        const bool fixed[3] = {bc.x != 255, bc.y != 255, bc.z != 255};
-        double vout[3];
-        const double im = 1.0 / mass;
-        for (int c = 0; c < 3; c++) {
-            if (fixed[c]) {
-                fb[c] = 0.0;
-                vout[c] = 0.0;
-            } else {
-                const double fdb = vbc[c] * dt * im;
-                mb += -vbc[c] * dt * fdc[c] * (im * im);
-                fb[c] = fdb * (1.0 - demf * sgnd(vpc[c]) * sgnd(fdc[c]));
-                vout[c] = vbc[c];
-            }
-        }
-        B.fbar[n] = make_double4(fb[0], fb[1], fb[2], mb);
-        vb = make_double4(vout[0], vout[1], vout[2], 0.0);
-    }
-    B.xbar[n] = xb;
-    B.vbar[n] = vb;
-}
-
-// loss on the top surface (j = nny - 1): per node w_v (v_y - tv)^2 + w_h (y - ty)^2,
-// its gradient seeds the adjoints; every other node's adjoint starts at zero
-__global__ void k_adj_loss(Mesh m, const double4* pos, const double4* vel, const double* tv, const double* ty,
-                           double wv, double wh, double* terms, AdjBufs B) {
-    long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= m.nn) return;
-    int i, j, k;
-    split3(n, m.nnx, m.nny, i, j, k);
-    double4 xb = make_double4(0, 0, 0, 0), vb = make_double4(0, 0, 0, 0);
-    if (j == m.nny - 1) {
-        long long t = (long long)i + (long long)k * m.nnx;
-        const double dv_ = vel[n].y - tv[t], dy = pos[n].y - ty[t];
-        terms[t] = wv * dv_ * dv_ + wh * dy * dy;
-        vb.y = 2.0 * wv * dv_;
-        xb.y = 2.0 * wh * dy;
-    }
-    B.xbar[n] = xb;
-    B.vbar[n] = vb;
-    B.fbar[n] = make_double4(0, 0, 0, 0);
-}
-
-// up to 6 array copies in one launch (checkpoint save / restore), 64-bit words
-struct CopyJob {
-    unsigned long long* dst[7];
-    const unsigned long long* src[7];
-    long long n[7];
-    int count;
-};
-__global__ void __launch_bounds__(256) k_copy_many(CopyJob J) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (int a = 0; a < J.count; a++) {
-        unsigned long long* d = J.dst[a];
-        const unsigned long long* s = J.src[a];
-        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < J.n[a]; i += stride) d[i] = s[i];
-    }
-}
-
-// per-element gradients: sum of the element's 10 tets in tet order
-__global__ void k_adj_reduce(long long ne, const double* pbar, double* gc, double* gf, double* gv) {
-    long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= ne) return;
-    double a = 0, b = 0, c = 0;
-    for (int t = 0; t < NT; t++) {
-        a += pbar[(e * NT + t) * 3 + 0];
-        b += pbar[(e * NT + t) * 3 + 1];
-        c += pbar[(e * NT + t) * 3 + 2];
-    }
-    gc[e] = a;
-    gf[e] = b;
-    gv[e] = c;
-}
-
 }  // namespace snac

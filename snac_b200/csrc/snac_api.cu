@@ -22,11 +22,10 @@
 #include <vector>
 
 #include "snac_gpu.h"
-#include "snac_adjoint.cuh"
-#include "snac_batch.cuh"
+#include "snac_kernels_api.cuh"
+#include "snac_launch.cuh"
 #include "snac_output.cuh"
 #include "snac_slab_plan.h"
-#include "snac_kernels.cuh"
 
 using namespace snac;
 
@@ -308,19 +307,6 @@ constexpr int force_rows(int dt_type, bool vonly) {
 #define MINLS_TET 8
 #endif
 constexpr int MINLS_TET_BLOCKS_PER_SM = MINLS_TET;
-// Raises a kernel's limit of dynamic shared memory to `most`, the largest size
-// that any launch of it asks for.  The limit belongs to the kernel on a
-// device, not to a handle: were it set to what each launch needs, one thread
-// could lower it between another's call and launch.  So it takes one value only.
-template <auto KERNEL>
-cudaError_t allow_smem(int device, size_t most) {
-    static std::atomic<unsigned long long> done{0};  // devices 0 to 63
-    const unsigned long long bit = device < 64 ? 1ull << device : 0ull;
-    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
-    return e;
-}
 // of a node gather: its most stages
 constexpr size_t most_stages(int rows) { return GATHER_STAGES * gather_stage_bytes(rows, NODE_THREADS); }
 static_assert(most_stages(CCHUNK) <= 227 * 1024, "the widest gather's stages fit an SM");
@@ -343,44 +329,14 @@ int launch_check_named(snac_gpu* h, const char* name) {
 // non-positive criterion lets the edge copy run with topoGradMax = 0
 bool topo_on(const Config& c) { return c.topo_kappa > 0 || !(c.topo_crit > 0); }
 
-template <int P>
-void launch_stress(snac_gpu* h, const Fields& F, const Config& c) {
-    if (h->mat)
-        k_calc_stresses<P, false><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c);
-    else
-        k_calc_stresses<P, true><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c);
-}
-template <int P>
-void launch_update(snac_gpu* h, const Fields& F, const Config& c, int pending) {
-    k_update_elements<P><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c, pending);
-}
-template <int P>
-void launch_fused(snac_gpu* h, const Fields& F, const Config& c) {
-    if (h->mat)
-        k_fused_step<P, false><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c);
-    else
-        k_fused_step<P, true><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c);
-}
+ElemGrid elem_grid(const snac_gpu* h) { return {elem_blocks(h->mesh), h->stream}; }
 // count_step: this launch opens the step (timeStep++, currentTime += dt)
 int op_energy_elements(snac_gpu* h, int count_step = 0) {
     if (!h->temperature) return 0;
-    if (h->mat)
-        k_heat_flux<false><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, fields(h), h->cfg,
-                                                                                   count_step);
-    else
-        k_heat_flux<true><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, fields(h), h->cfg,
-                                                                                  count_step);
+    run_heat_flux(elem_grid(h), !h->mat, h->mesh, fields(h), h->cfg, count_step);
     h->launches++;
     if (count_step) h->time_step++;
     return launch_check_named(h, "k_heat_flux");
-}
-
-template <int P>
-void launch_fused_stress(snac_gpu* h, const Fields& F, const Config& c) {
-    if (h->mat)
-        k_fused_stress<P, false><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c);
-    else
-        k_fused_stress<P, true><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c);
 }
 
 // temperature runs: the pending element update of the previous step with
@@ -390,15 +346,15 @@ int op_fused_stress(snac_gpu* h) {
     Config c = h->cfg;
     c.time_step_zero = 0;
     switch (h->constitutive) {
-        case SNAC_RHEOLOGY_ELASTIC: launch_fused_stress<SNAC_RHEOLOGY_ELASTIC>(h, F, c); break;
-        case SNAC_RHEOLOGY_PLASTIC: launch_fused_stress<SNAC_RHEOLOGY_PLASTIC>(h, F, c); break;
+        case SNAC_RHEOLOGY_ELASTIC: run_fused_stress<SNAC_RHEOLOGY_ELASTIC>(elem_grid(h), !h->mat, h->mesh, F, c); break;
+        case SNAC_RHEOLOGY_PLASTIC: run_fused_stress<SNAC_RHEOLOGY_PLASTIC>(elem_grid(h), !h->mat, h->mesh, F, c); break;
         case SNAC_RHEOLOGY_VISCOPLASTIC:
             if (h->dp)
-                launch_fused_stress<SNAC_VP_DP>(h, F, c);
+                run_fused_stress<SNAC_VP_DP>(elem_grid(h), !h->mat, h->mesh, F, c);
             else
-                launch_fused_stress<SNAC_RHEOLOGY_VISCOPLASTIC>(h, F, c);
+                run_fused_stress<SNAC_RHEOLOGY_VISCOPLASTIC>(elem_grid(h), !h->mat, h->mesh, F, c);
             break;
-        case SNAC_RHEOLOGY_MAXWELL: launch_fused_stress<SNAC_RHEOLOGY_MAXWELL>(h, F, c); break;
+        case SNAC_RHEOLOGY_MAXWELL: run_fused_stress<SNAC_RHEOLOGY_MAXWELL>(elem_grid(h), !h->mat, h->mesh, F, c); break;
     }
     h->launches++;
     return launch_check_named(h, "k_fused_stress");
@@ -417,15 +373,15 @@ int op_energy_nodes(snac_gpu* h, int count_step = 0) {
 int op_calc_stresses(snac_gpu* h) {
     Fields F = fields(h);
     switch (h->constitutive) {
-        case SNAC_RHEOLOGY_ELASTIC: launch_stress<SNAC_RHEOLOGY_ELASTIC>(h, F, h->cfg); break;
-        case SNAC_RHEOLOGY_PLASTIC: launch_stress<SNAC_RHEOLOGY_PLASTIC>(h, F, h->cfg); break;
+        case SNAC_RHEOLOGY_ELASTIC: run_calc_stresses<SNAC_RHEOLOGY_ELASTIC>(elem_grid(h), !h->mat, h->mesh, F, h->cfg); break;
+        case SNAC_RHEOLOGY_PLASTIC: run_calc_stresses<SNAC_RHEOLOGY_PLASTIC>(elem_grid(h), !h->mat, h->mesh, F, h->cfg); break;
         case SNAC_RHEOLOGY_VISCOPLASTIC:
             if (h->dp)
-                launch_stress<SNAC_VP_DP>(h, F, h->cfg);
+                run_calc_stresses<SNAC_VP_DP>(elem_grid(h), !h->mat, h->mesh, F, h->cfg);
             else
-                launch_stress<SNAC_RHEOLOGY_VISCOPLASTIC>(h, F, h->cfg);
+                run_calc_stresses<SNAC_RHEOLOGY_VISCOPLASTIC>(elem_grid(h), !h->mat, h->mesh, F, h->cfg);
             break;
-        case SNAC_RHEOLOGY_MAXWELL: launch_stress<SNAC_RHEOLOGY_MAXWELL>(h, F, h->cfg); break;
+        case SNAC_RHEOLOGY_MAXWELL: run_calc_stresses<SNAC_RHEOLOGY_MAXWELL>(elem_grid(h), !h->mat, h->mesh, F, h->cfg); break;
     }
     h->launches++;
     return launch_check_named(h, "k_calc_stresses");
@@ -464,8 +420,8 @@ int op_update_elements(snac_gpu* h, bool step_zero, int pending = 0) {
     Config c = h->cfg;
     c.time_step_zero = step_zero ? 1 : 0;
     switch (h->constitutive) {
-        case SNAC_RHEOLOGY_MAXWELL: launch_update<SNAC_RHEOLOGY_MAXWELL>(h, F, c, pending); break;
-        default: launch_update<SNAC_RHEOLOGY_ELASTIC>(h, F, c, pending); break;
+        case SNAC_RHEOLOGY_MAXWELL: run_update_elements<SNAC_RHEOLOGY_MAXWELL>(elem_grid(h), h->mesh, F, c, pending); break;
+        default: run_update_elements<SNAC_RHEOLOGY_ELASTIC>(elem_grid(h), h->mesh, F, c, pending); break;
     }
     h->launches++;
     return launch_check_named(h, "k_update_elements");
@@ -478,15 +434,15 @@ int op_fused(snac_gpu* h) {
     Config c = h->cfg;
     c.time_step_zero = 0;
     switch (h->constitutive) {
-        case SNAC_RHEOLOGY_ELASTIC: launch_fused<SNAC_RHEOLOGY_ELASTIC>(h, F, c); break;
-        case SNAC_RHEOLOGY_PLASTIC: launch_fused<SNAC_RHEOLOGY_PLASTIC>(h, F, c); break;
+        case SNAC_RHEOLOGY_ELASTIC: run_fused_step<SNAC_RHEOLOGY_ELASTIC>(elem_grid(h), !h->mat, h->mesh, F, c); break;
+        case SNAC_RHEOLOGY_PLASTIC: run_fused_step<SNAC_RHEOLOGY_PLASTIC>(elem_grid(h), !h->mat, h->mesh, F, c); break;
         case SNAC_RHEOLOGY_VISCOPLASTIC:
             if (h->dp)
-                launch_fused<SNAC_VP_DP>(h, F, c);
+                run_fused_step<SNAC_VP_DP>(elem_grid(h), !h->mat, h->mesh, F, c);
             else
-                launch_fused<SNAC_RHEOLOGY_VISCOPLASTIC>(h, F, c);
+                run_fused_step<SNAC_RHEOLOGY_VISCOPLASTIC>(elem_grid(h), !h->mat, h->mesh, F, c);
             break;
-        case SNAC_RHEOLOGY_MAXWELL: launch_fused<SNAC_RHEOLOGY_MAXWELL>(h, F, c); break;
+        case SNAC_RHEOLOGY_MAXWELL: run_fused_step<SNAC_RHEOLOGY_MAXWELL>(elem_grid(h), !h->mat, h->mesh, F, c); break;
     }
     h->launches++;
     h->time_step++;
@@ -495,12 +451,7 @@ int op_fused(snac_gpu* h) {
 
 int op_min_length_scale_sync(snac_gpu* h) {
     if (h->temperature) {  // with the heat flux of the next step
-        if (h->mat)
-            k_heat_flux_min_length_scale<false><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(
-                h->mesh, fields(h), h->cfg);
-        else
-            k_heat_flux_min_length_scale<true><<<elem_blocks(h->mesh), ELEM_WARPS * 32, 0, h->stream>>>(
-                h->mesh, fields(h), h->cfg);
+        run_heat_flux_min_length_scale(elem_grid(h), !h->mat, h->mesh, fields(h), h->cfg);
         h->launches++;
         int rc = launch_check_named(h, "k_heat_flux_min_length_scale");
         if (rc) return rc;
@@ -780,24 +731,16 @@ int node_out(snac_gpu* h, const double4* src, double* dst, int what) {
 // node slabs block ranges of the node launch; an empty range launches nothing.
 int op_calc_stresses_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     if (b1 <= b0) return 0;
-    const unsigned nb = (unsigned)(b1 - b0);
-    const Config& c = h->cfg;
-    cudaStream_t st = h->stream;
-#define SLAB_STRESS(P)                                                                              \
-    do {                                                                                             \
-        if (h->mat) k_calc_stresses_slab<P, false><<<nb, ELEM_WARPS * 32, 0, st>>>(h->mesh, F, c, b0); \
-        else k_calc_stresses_slab<P, true><<<nb, ELEM_WARPS * 32, 0, st>>>(h->mesh, F, c, b0);         \
-    } while (0)
+    const ElemGrid g{(unsigned)(b1 - b0), h->stream};
     switch (h->constitutive) {
-        case SNAC_RHEOLOGY_ELASTIC: SLAB_STRESS(SNAC_RHEOLOGY_ELASTIC); break;
-        case SNAC_RHEOLOGY_PLASTIC: SLAB_STRESS(SNAC_RHEOLOGY_PLASTIC); break;
+        case SNAC_RHEOLOGY_ELASTIC: run_calc_stresses_slab<SNAC_RHEOLOGY_ELASTIC>(g, !h->mat, h->mesh, F, h->cfg, b0); break;
+        case SNAC_RHEOLOGY_PLASTIC: run_calc_stresses_slab<SNAC_RHEOLOGY_PLASTIC>(g, !h->mat, h->mesh, F, h->cfg, b0); break;
         case SNAC_RHEOLOGY_VISCOPLASTIC:
-            if (h->dp) SLAB_STRESS(SNAC_VP_DP);
-            else SLAB_STRESS(SNAC_RHEOLOGY_VISCOPLASTIC);
+            if (h->dp) run_calc_stresses_slab<SNAC_VP_DP>(g, !h->mat, h->mesh, F, h->cfg, b0);
+            else run_calc_stresses_slab<SNAC_RHEOLOGY_VISCOPLASTIC>(g, !h->mat, h->mesh, F, h->cfg, b0);
             break;
-        case SNAC_RHEOLOGY_MAXWELL: SLAB_STRESS(SNAC_RHEOLOGY_MAXWELL); break;
+        case SNAC_RHEOLOGY_MAXWELL: run_calc_stresses_slab<SNAC_RHEOLOGY_MAXWELL>(g, !h->mat, h->mesh, F, h->cfg, b0); break;
     }
-#undef SLAB_STRESS
     h->launches++;
     return launch_check_named(h, "k_calc_stresses_slab");
 }
@@ -830,24 +773,20 @@ int op_loop_nodes_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
 
 int op_update_elements_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     if (b1 <= b0) return 0;
-    const unsigned nb = (unsigned)(b1 - b0);
+    const ElemGrid g{(unsigned)(b1 - b0), h->stream};
     Config c = h->cfg;
     c.time_step_zero = 0;
     if (h->constitutive == SNAC_RHEOLOGY_MAXWELL)
-        k_update_elements_slab<SNAC_RHEOLOGY_MAXWELL><<<nb, ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c, b0);
+        run_update_elements_slab<SNAC_RHEOLOGY_MAXWELL>(g, h->mesh, F, c, b0);
     else
-        k_update_elements_slab<SNAC_RHEOLOGY_ELASTIC><<<nb, ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, c, b0);
+        run_update_elements_slab<SNAC_RHEOLOGY_ELASTIC>(g, h->mesh, F, c, b0);
     h->launches++;
     return launch_check_named(h, "k_update_elements_slab");
 }
 
 int op_heat_flux_slab(snac_gpu* h, const Fields& F, int b0, int b1) {
     if (b1 <= b0) return 0;
-    const unsigned nb = (unsigned)(b1 - b0);
-    if (h->mat)
-        k_heat_flux_slab<false><<<nb, ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, h->cfg, b0);
-    else
-        k_heat_flux_slab<true><<<nb, ELEM_WARPS * 32, 0, h->stream>>>(h->mesh, F, h->cfg, b0);
+    run_heat_flux_slab({(unsigned)(b1 - b0), h->stream}, !h->mat, h->mesh, F, h->cfg, b0);
     h->launches++;
     return launch_check_named(h, "k_heat_flux_slab");
 }
@@ -1981,7 +1920,7 @@ int bcheck_launch(snac_gpu_batch* b, const char* name) {
 template <int OP>
 int blaunch_elem(snac_gpu_batch* b, const ModelDesc* D, const snac_gpu_batch::List& L) {
     if (L.n == 0) return 0;
-    kb_elements<OP><<<tile_grid(b, L.n, b->tune.elem_blocks_per_sm), ELEM_WARPS * 32, 0, b->stream>>>(D, b->tiles + L.off, L.n);
+    run_tiles<OP>({tile_grid(b, L.n, b->tune.elem_blocks_per_sm), b->stream}, D, b->tiles + L.off, L.n);
     return bcheck_launch(b, "kb_elements");
 }
 
@@ -1997,17 +1936,19 @@ int blaunch_nodes(snac_gpu_batch* b, const ModelDesc* D, const snac_gpu_batch::L
 template <int OP, int P, int TEMP>
 int blaunch_elem_c(snac_gpu_batch* b, const ModelDesc* D, const snac_gpu_batch::List& L) {
     if (L.n == 0) return 0;
-    kb_elements_c<OP, P, TEMP><<<tile_grid(b, L.n, b->tune.elem_blocks_per_sm), ELEM_WARPS * 32, 0, b->stream>>>(
-        D, b->tiles + L.off, L.n);
+    // the heat flux is the same kernel for every hook
+    constexpr bool heat = OP == BOP_HEAT_FLUX || (OP == BOP_FUSED && TEMP);
+    run_class_tiles<OP, heat ? SNAC_RHEOLOGY_ELASTIC : P, TEMP>(
+        {tile_grid(b, L.n, b->tune.elem_blocks_per_sm), b->stream}, D, b->tiles + L.off, L.n);
     return bcheck_launch(b, "kb_elements_c");
 }
 
-// one launch per rheology class present; temp_only skips the classes without temperature
+// one launch per rheology class present (two of the operations are for models with temperature only)
 template <int OP>
-int blaunch_elem_classes(snac_gpu_batch* b, const ModelDesc* D, bool temp_only) {
+int blaunch_elem_classes(snac_gpu_batch* b, const ModelDesc* D) {
     int rc = 0;
     const auto& C = b->elem_cls;
-    if (!temp_only) {
+    if constexpr (OP == BOP_FUSED || OP == BOP_STRESS) {
         if (!rc) rc = blaunch_elem_c<OP, SNAC_RHEOLOGY_ELASTIC, 0>(b, D, C[0]);
         if (!rc) rc = blaunch_elem_c<OP, SNAC_RHEOLOGY_PLASTIC, 0>(b, D, C[2]);
     }
@@ -2025,12 +1966,12 @@ int record_batch_step(snac_gpu_batch* b, bool fused, int parity) {
     int rc;
     const bool by_class = b->tune.split_classes != 0;
     if (fused) {
-        if ((rc = by_class ? blaunch_elem_classes<BOP_FUSED>(b, D, false) : blaunch_elem<BOP_FUSED>(b, D, b->elem_all)))
+        if ((rc = by_class ? blaunch_elem_classes<BOP_FUSED>(b, D) : blaunch_elem<BOP_FUSED>(b, D, b->elem_all)))
             return rc;
     } else {
         kb_begin_step<<<mb, 128, 0, b->stream>>>(D, b->n);
         if ((rc = bcheck_launch(b, "kb_begin_step"))) return rc;
-        if ((rc = by_class ? blaunch_elem_classes<BOP_HEAT_FLUX>(b, D, true)
+        if ((rc = by_class ? blaunch_elem_classes<BOP_HEAT_FLUX>(b, D)
                            : blaunch_elem<BOP_HEAT_FLUX>(b, D, b->elem_temp)))
             return rc;
     }
@@ -2038,10 +1979,10 @@ int record_batch_step(snac_gpu_batch* b, bool fused, int parity) {
     // temperature models: after the energy hooks, the pending element update
     // fused with the stress update (fused step) or the stress update alone
     if (fused)
-        rc = by_class ? blaunch_elem_classes<BOP_FUSED_STRESS>(b, D, true)
+        rc = by_class ? blaunch_elem_classes<BOP_FUSED_STRESS>(b, D)
                       : blaunch_elem<BOP_FUSED_STRESS>(b, D, b->elem_temp);
     else
-        rc = by_class ? blaunch_elem_classes<BOP_STRESS>(b, D, false) : blaunch_elem<BOP_STRESS>(b, D, b->elem_all);
+        rc = by_class ? blaunch_elem_classes<BOP_STRESS>(b, D) : blaunch_elem<BOP_STRESS>(b, D, b->elem_all);
     if (rc) return rc;
     if ((rc = blaunch_nodes<BOP_LOOP_NODES>(b, D, b->node_all, b->tune.node_threads))) return rc;
     // the node loop wrote the new coordinates into the other buffer
@@ -2486,25 +2427,15 @@ int adjoint_supported(snac_gpu* h) {
     return 0;
 }
 
-template <int P>
-int adj_tet_launch_p(snac_gpu* h, const Fields& F, const AdjState& S, const AdjBufs& B, int rotate, int first_rev,
-                     double dt) {
-    CK(allow_smem<k_adj_tet<P>>(h->device, sizeof(AdjSmem)));
-    k_adj_tet<P><<<elem_blocks(h->mesh), ELEM_WARPS * 32, sizeof(AdjSmem), h->stream>>>(h->mesh, F, h->cfg, S, B, rotate,
-                                                                                       first_rev, dt);
-    return 0;
-}
-
 int adj_tet_launch(snac_gpu* h, const AdjState& S, const AdjBufs& B, int rotate, int first_rev, double dt) {
     const Fields F = fields(h);
-    int rc;
+    const auto run = [&](auto f) { return f(h->device, elem_grid(h), h->mesh, F, h->cfg, S, B, rotate, first_rev, dt); };
     switch (h->constitutive) {
-        case SNAC_RHEOLOGY_ELASTIC: rc = adj_tet_launch_p<SNAC_RHEOLOGY_ELASTIC>(h, F, S, B, rotate, first_rev, dt); break;
-        case SNAC_RHEOLOGY_PLASTIC: rc = adj_tet_launch_p<SNAC_RHEOLOGY_PLASTIC>(h, F, S, B, rotate, first_rev, dt); break;
-        case SNAC_RHEOLOGY_MAXWELL: rc = adj_tet_launch_p<SNAC_RHEOLOGY_MAXWELL>(h, F, S, B, rotate, first_rev, dt); break;
-        default: rc = adj_tet_launch_p<SNAC_RHEOLOGY_VISCOPLASTIC>(h, F, S, B, rotate, first_rev, dt);
+        case SNAC_RHEOLOGY_ELASTIC: CK(run(run_adj_tet<SNAC_RHEOLOGY_ELASTIC>)); break;
+        case SNAC_RHEOLOGY_PLASTIC: CK(run(run_adj_tet<SNAC_RHEOLOGY_PLASTIC>)); break;
+        case SNAC_RHEOLOGY_MAXWELL: CK(run(run_adj_tet<SNAC_RHEOLOGY_MAXWELL>)); break;
+        default: CK(run(run_adj_tet<SNAC_RHEOLOGY_VISCOPLASTIC>));
     }
-    if (rc) return rc;
     h->launches++;
     return launch_check_named(h, "k_adj_tet");
 }

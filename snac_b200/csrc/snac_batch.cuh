@@ -212,33 +212,4 @@ __global__ void __launch_bounds__(NODE_TILE_MAX) kb_nodes(const ModelDesc* __res
     }
 }
 
-// _Snac_Context_Sync of every model: one thread per model
-__global__ void kb_sync(const ModelDesc* __restrict__ D, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) sync_one(D[i].cfg, D[i].F.sc, D[i].wave_speed);
-}
-
-// _AbstractContext_Execute_Hook of every model (a step that does not start
-// with the fused kernel): timeStep++ and dt = dtFactor * dt
-__global__ void kb_begin_step(const ModelDesc* __restrict__ D, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        DevScalars* sc = D[i].F.sc;
-        sc->time_step += 1;
-        sc->dt = 1.0 * sc->dt;
-        sc->current_time += sc->dt;
-    }
-}
-
-__global__ void kb_status(const ModelDesc* __restrict__ D, int n, ModelStatus* out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const DevScalars* sc = D[i].F.sc;
-        out[i].status = sc->status;
-        out[i].pad = 0;
-        out[i].err_index = sc->err_index;
-        out[i].time_step = sc->time_step;
-    }
-}
-
 }  // namespace snac

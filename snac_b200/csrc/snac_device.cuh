@@ -208,7 +208,7 @@ __host__ __device__ __forceinline__ bool positive_within(double y) {
 // code (with its own special-case paths) then is not inlined at each of the
 // few dozen division sites of an element kernel, where it cost registers and
 // instruction scheduling on the common path.
-__host__ __device__ __noinline__ double ieee_div(double x, double y) { return x / y; }
+inline __host__ __device__ __noinline__ double ieee_div(double x, double y) { return x / y; }
 
 // The correction step RN(q0 + r z), r = x - q0 y, written as
 // -RN(-r z - q0): the same value (round-to-nearest is symmetric), and for
@@ -747,7 +747,7 @@ __device__ __forceinline__ double tan_dil(const DevMaterial& m, double psi) {
 // is an uninitialised function-scope variable in the reference on its first
 // use; here it starts at 0.  IEEE division and square root throughout (a
 // rarely taken path).  Returns whether the tet yielded.
-__device__ __noinline__ bool dp_return_map(double s[6], double sd[3], const double S0[6], const double e[6],
+inline __device__ __noinline__ bool dp_return_map(double s[6], double sd[3], const double S0[6], const double e[6],
                                            double vic1, double vic2, double rmu, double bulkm, double qphi,
                                            double qpsi, double kphi, double st, double tol, int mite, double pst[6],
                                            double& eps_p) {
