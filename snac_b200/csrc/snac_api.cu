@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "snac_gpu.h"
+#include "snac_capture.h"
 #include "snac_kernels_api.cuh"
 #include "snac_launch.cuh"
 #include "snac_output.cuh"
@@ -583,26 +584,55 @@ void drop_graphs(snac_gpu* h) {
     for (auto& g : h->run_graph) drop(g);
 }
 
+// capture_graph's calls on a stream
+struct StreamCapture {
+    using Graph = cudaGraph_t;
+    using Exec = cudaGraphExec_t;
+    cudaStream_t stream;
+    cudaError_t error = cudaSuccess;  // of the call that failed
+    const char* call = "";
+    int check(cudaError_t e, const char* what) {
+        if (e == cudaSuccess) return 0;
+        error = e;
+        call = what;
+        return SNAC_GPU_ECUDA;
+    }
+    int begin() { return check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "graph capture"); }
+    int end(Graph* g) { return check(cudaStreamEndCapture(stream, g), "graph capture"); }
+    int instantiate(Exec* e, Graph g) { return check(cudaGraphInstantiate(e, g, 0), "graph instantiate"); }
+    void destroy(Graph g) { cudaGraphDestroy(g); }
+};
+// and a handle's bookkeeping that recording a step advances
+struct HandleCapture : StreamCapture {
+    struct Mark {
+        long long launches, time_step;
+        int parity;
+    };
+    snac_gpu* h;
+    explicit HandleCapture(snac_gpu* h_) : StreamCapture{h_->stream}, h(h_) {}
+    Mark mark() const { return {h->launches, h->time_step, h->parity}; }
+    void restore(const Mark& m) { h->launches = m.launches, h->time_step = m.time_step, h->parity = m.parity; }
+    long long launched_since(const Mark& m) const { return h->launches - m.launches; }
+};
+// n steps as one graph of the handle
+int capture_steps(snac_gpu* h, int n, bool fused, cudaGraphExec_t* out, int* kernels) {
+    HandleCapture api(h);
+    int recorded = 0;  // a step that cannot be recorded sets its own message
+    const auto record = [&] {
+        for (int s = 0; s < n && !recorded; s++) recorded = record_step(h, fused);
+        return recorded;
+    };
+    const int rc = capture_graph(api, record, out, kernels);
+    return rc && !recorded ? set_err(h, rc, -1, "%s: %s", api.call, cudaGetErrorString(api.error)) : rc;
+}
+
 // one step from the handle's CUDA graph for its (pending, parity) state,
 // captured on first use; no status read
 int launch_step(snac_gpu* h) {
     if (int rc = request_scalars(h, h->time_step + 1)) return rc;
     int p = h->parity, f = h->pending ? 1 : 0, r = (h->temperature && h->hflux_ready) ? 1 : 0;
-    if (!h->graph[r][f][p]) {
-        cudaGraph_t g;
-        long long l0 = h->launches, ts0 = h->time_step;
-        CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = record_step(h, f == 1);
-        cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-        if (rc) return rc;
-        if (e != cudaSuccess) return set_err(h, SNAC_GPU_ECUDA, -1, "graph capture: %s", cudaGetErrorString(e));
-        CK(cudaGraphInstantiate(&h->graph[r][f][p], g, 0));
-        cudaGraphDestroy(g);
-        h->steps_kernels[r][f] = (int)(h->launches - l0);
-        h->launches = l0;  // counted again below, when the graph actually runs
-        h->time_step = ts0;
-        h->parity = p;
-    }
+    if (!h->graph[r][f][p])
+        if (int rc = capture_steps(h, 1, f == 1, &h->graph[r][f][p], &h->steps_kernels[r][f])) return rc;
     CK(cudaGraphLaunch(h->graph[r][f][p], h->stream));
     h->launches += h->steps_kernels[r][f];
     h->time_step++;
@@ -630,22 +660,7 @@ int run_steps(snac_gpu* h, int n) {
             continue;
         }
         cudaGraphExec_t& ge = h->run_graph[h->parity];
-        if (!ge) {
-            cudaGraph_t g;
-            const long long l0 = h->launches, ts0 = h->time_step;
-            CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-            rc = 0;
-            for (int s = 0; s < RUN_STEPS && !rc; s++) rc = record_step(h, true);
-            cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-            h->run_kernels = (int)(h->launches - l0);
-            h->launches = l0;  // counted when the graph runs
-            h->time_step = ts0;
-            if (rc) return rc;
-            if (e != cudaSuccess) return set_err(h, SNAC_GPU_ECUDA, -1, "graph capture: %s", cudaGetErrorString(e));
-            e = cudaGraphInstantiate(&ge, g, 0);
-            cudaGraphDestroy(g);
-            if (e != cudaSuccess) return set_err(h, SNAC_GPU_ECUDA, -1, "graph instantiate: %s", cudaGetErrorString(e));
-        }
+        if (!ge && (rc = capture_steps(h, RUN_STEPS, true, &ge, &h->run_kernels))) return rc;
         CK(cudaGraphLaunch(ge, h->stream));
         h->launches += h->run_kernels;
         h->time_step += RUN_STEPS;
@@ -2017,6 +2032,16 @@ int batch_prepare(snac_gpu_batch* b, bool* fused) {
     return 0;
 }
 
+// capture_graph's calls and the batch's count of launches
+struct BatchCapture : StreamCapture {
+    using Mark = long long;
+    snac_gpu_batch* b;
+    explicit BatchCapture(snac_gpu_batch* b_) : StreamCapture{b_->stream}, b(b_) {}
+    Mark mark() const { return b->launches; }
+    void restore(Mark m) { b->launches = m; }
+    long long launched_since(Mark m) const { return b->launches - m; }
+};
+
 // launches nsteps batched steps (no status read)
 int batch_run(snac_gpu_batch* b, int nsteps) {
     bool fused;
@@ -2034,19 +2059,14 @@ int batch_run(snac_gpu_batch* b, int nsteps) {
         const int k = chunk ? S : 1;
         cudaGraphExec_t& ge = b->graph[chunk][b->parity];
         if (!ge) {
-            cudaGraph_t g;
-            long long l0 = b->launches;
-            BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-            int rc2 = 0;
-            for (int j = 0; j < k && !rc2; j++) rc2 = record_batch_step(b, true, b->parity ^ (j & 1));
-            cudaError_t e = cudaStreamEndCapture(b->stream, &g);
-            if (rc2) return rc2;
-            if (e != cudaSuccess) return bset_err(b, SNAC_GPU_ECUDA, -1, "graph capture: %s", cudaGetErrorString(e));
-            e = cudaGraphInstantiate(&ge, g, 0);
-            cudaGraphDestroy(g);
-            if (e != cudaSuccess) return bset_err(b, SNAC_GPU_ECUDA, -1, "graph instantiate: %s", cudaGetErrorString(e));
-            b->graph_kernels[chunk] = (int)(b->launches - l0);
-            b->launches = l0;
+            BatchCapture api(b);
+            int recorded = 0;
+            const auto record = [&] {
+                for (int j = 0; j < k && !recorded; j++) recorded = record_batch_step(b, true, b->parity ^ (j & 1));
+                return recorded;
+            };
+            rc = capture_graph(api, record, &ge, &b->graph_kernels[chunk]);
+            if (rc) return recorded ? rc : bset_err(b, rc, -1, "%s: %s", api.call, cudaGetErrorString(api.error));
         }
         BCK(cudaGraphLaunch(ge, b->stream));
         b->launches += b->graph_kernels[chunk];
