@@ -367,6 +367,14 @@ int  snac_gpu_fp64_rate(double* fma_per_second);
  * signed zeros, exact quotients and ties) compared bit for bit with the
  * IEEE quotient of the GPU; *mismatches receives the count (expected 0). */
 int  snac_gpu_selftest_division(long long n, unsigned long long seed, long long* mismatches);
+/* Self-test of the bounded wait of the node gathers (csrc/snac_kernels.cuh):
+ * one block gathers a mesh of 3x2x3 hexes twice, with 1, 2 or 4 stages.  The
+ * pair of hexes `late` (0 to 3; another value: none) never completes, so its wait runs
+ * out after limit_ms (0 to 1000).  *status receives SNAC_GPU_OK or
+ * SNAC_GPU_ETIMEDOUT, counts[0] and [1] the threads whose first and second
+ * gather succeeded (64 each if none is late; the second is given up at once
+ * after a failure), counts[2] the hexes that the first one added. */
+int  snac_gpu_selftest_gather(int stages, int late, double limit_ms, int* status, int counts[3]);
 
 /* ---- adjoint ------------------------------------------------------------------
  * No counterpart in the reference.  Loss on the top surface (node plane

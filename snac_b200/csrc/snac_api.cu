@@ -895,6 +895,35 @@ double hydrostatic_ic(const snac_gpu_desc* d, const std::vector<double>& coord, 
 
 extern "C" {
 
+int snac_gpu_selftest_gather(int stages, int late, double limit_ms, int* status, int counts[3]) {
+    if (!status || !counts || (stages != 1 && stages != 2 && stages != 4) || !(limit_ms >= 0.0 && limit_ms <= 1000.0))
+        return SNAC_GPU_EINVAL;
+    Mesh m{};
+    m.nx = 3, m.ny = 2, m.nz = 3;  // 48 nodes: one block
+    m.nnx = m.nx + 1, m.nny = m.ny + 1, m.nnz = m.nz + 1;
+    m.ne = (long long)m.nx * m.ny * m.nz;
+    m.nn = (long long)m.nnx * m.nny * m.nnz;
+    const size_t bytes = (size_t)((m.ne + GROUP - 1) / GROUP) * HROWS * GROUP * sizeof(double);
+    const size_t smem = stages * gather_stage_bytes(HEAT_CHUNK + HEAT_TAIL, NODE_THREADS);
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return SNAC_GPU_ENODEV;
+    char* d = nullptr;  // the groups, then the counts
+    if (cudaMalloc(&d, bytes + 3 * sizeof(int)) != cudaSuccess) return SNAC_GPU_ENOMEM;
+    int* const out = reinterpret_cast<int*>(d + bytes);
+    cudaError_t e = cudaMemset(d, 0, bytes + 3 * sizeof(int));
+    if (e == cudaSuccess) e = allow_smem<k_selftest_gather>(dev, most_stages(HEAT_CHUNK + HEAT_TAIL));
+    if (e == cudaSuccess) {
+        k_selftest_gather<<<1, NODE_THREADS, smem>>>(m, reinterpret_cast<const double*>(d), stages, late,
+                                                     (unsigned long long)(limit_ms * 1.0e6), out);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(counts, out, 3 * sizeof(int), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return SNAC_GPU_ECUDA;
+    *status = counts[0] == NODE_THREADS ? SNAC_GPU_OK : SNAC_GPU_ETIMEDOUT;
+    return 0;
+}
+
 int snac_gpu_selftest_division(long long n, unsigned long long seed, long long* mismatches) {
     if (!mismatches || n < 0) return SNAC_GPU_EINVAL;
     unsigned long long* d = nullptr;

@@ -189,6 +189,7 @@ __global__ void __launch_bounds__(NODE_TILE_MAX) kb_nodes(const ModelDesc* __res
     Tiles T(D, tiles, ntiles);
     for (int i = blockIdx.x; i < ntiles; i += gridDim.x, phase ^= 1) {
         const int b = T.at(i, md);
+        if (OP != BOP_MINLS && S.gave_up) break;  // (T.at is a barrier: the whole block sees the same)
         if (OP == BOP_LOOP_NODES) {
             const bool vo = md.cfg.vonly != 0;
             switch (md.cfg.dt_type) {

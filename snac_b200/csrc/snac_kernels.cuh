@@ -1275,8 +1275,36 @@ __device__ __forceinline__ double node_update(const Mesh& m, const Fields& F, co
 struct GatherSmem {
     unsigned long long full[4];  // mbarrier of each pair
     int g0[4], ng[4];            // first group and number of groups of each pair
+    int gave_up;                 // a pair did not arrive in time: the block gathers no further tile
 };
 extern __shared__ __align__(16) unsigned char g_gather[];
+
+// Waits for the phase of parity `phase` of an mbarrier, false if it has not
+// completed after `limit` ns of the device's clock.  The usual wait ends
+// within a few tries, each of which may suspend the thread for a time of the
+// hardware's choosing; the clock is read, and the barrier only tested, after those.
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ bool mbarrier_wait(unsigned bar, unsigned phase, unsigned long long limit) {
+    unsigned done;
+    for (int tries = 0; tries < 32; tries++) {
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(phase) : "memory");
+        if (done) return true;
+    }
+    for (const unsigned long long t0 = global_ns(); global_ns() - t0 < limit;) {
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(phase) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+constexpr unsigned long long GATHER_LIMIT = 1000000000ull;  // ns
 
 template <int CHUNK, int TAIL>  // rows of a pair's chunk; rows after the four chunks
 struct Gather {
@@ -1285,6 +1313,7 @@ struct Gather {
     const double* src;   // the groups
     int frows, stages, stage_entries;
     unsigned phase;      // parity of the mbarriers (blocks that take several tiles use them again)
+    unsigned long long limit = GATHER_LIMIT;  // of the wait for a pair
 
     __device__ __forceinline__ double* stage(int c) const {
         return reinterpret_cast<double*>(g_gather) + (c % stages) * stage_entries;
@@ -1316,31 +1345,27 @@ struct Gather {
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          smem_addr(d)), "l"(s), "r"(bytes), "r"(bar) : "memory");
     }
-    // false if the copies have not arrived after about a second
-    __device__ __forceinline__ bool wait(int c) const {
-        const unsigned bar = smem_addr(&S.full[c]);
-        for (int tries = 0; tries < (1 << 20); tries++) {
-            unsigned done;
-            asm volatile("{\n\t.reg .pred p;\n\t"
-                         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                         "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(phase) : "memory");
-            if (done) return true;
-        }
-        return false;
-    }
+    __device__ __forceinline__ bool wait(int c) const { return mbarrier_wait(smem_addr(&S.full[c]), phase, limit); }
     // Runs add(ne, base) for the hexes ne = 0..7 of node (i, j, k) in the reference's order
     // (HexaEL.c:529-573: pair by pair, i - 1 before i; absent hexes are
     // skipped, Force.c:92), base the hex's entry of row 0 of pair c's stage.
+    // False in the threads for which a pair has not arrived within the limit: they
+    // add nothing from it on, and warp 0 then fetches no more (so that the other
+    // warps' waits run out too).
     template <class Add>
     __device__ __forceinline__ bool run(const Mesh& m, int lb, bool active, int i, int j, int k, Add&& add) const {
         plan(m, lb);
         __syncthreads();
         if (threadIdx.x < 32)
             for (int c = 0; c < stages; c++) fetch(c);
+        int fetched = stages;
         bool ok = true;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            ok = wait(c) & ok;
+            if (ok && !wait(c)) {
+                ok = false;
+                S.gave_up = 1;
+            }
             const int ej = j - 1 + (c & 1), ek = k - 1 + (c >> 1);
             if (ok && active && ej >= 0 && ej < m.ny && ek >= 0 && ek < m.nz) {
                 const int row = (ej + ek * m.ny) * m.nx, g0 = S.g0[c] * GROUP;
@@ -1355,9 +1380,15 @@ struct Gather {
             }
             if (c + stages < 4) {
                 __syncthreads();
-                if (threadIdx.x < 32) fetch(c + stages);
+                if (threadIdx.x < 32 && __all_sync(FULL, ok)) {
+                    fetch(c + stages);
+                    fetched++;
+                }
             }
         }
+        // the block stays until its copies have arrived, or the limit has passed again
+        if (!ok && threadIdx.x < 32)
+            for (int c = 0; c < fetched; c++) wait(c);
         return ok;
     }
 };
@@ -1367,6 +1398,7 @@ __device__ __forceinline__ void gather_init(GatherSmem& S) {
 #pragma unroll
         for (int c = 0; c < 4; c++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&S.full[c])) : "memory");
+        S.gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
 }

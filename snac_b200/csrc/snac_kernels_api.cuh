@@ -225,6 +225,34 @@ __global__ void k_selftest_division(long long n, unsigned long long seed, unsign
     if (local) atomicAdd(bad, local);
 }
 
+// ---- self-test of the gather's bounded wait ---------------------------------------------
+// One block gathers a small mesh's heat groups twice, with `stages` stages and
+// `limit` ns for each wait.  The barrier of pair `late` (none if it is not 0 to 3) is
+// told to expect 16 bytes more than the copies bring: that pair never completes,
+// although every copy arrives.  out: threads whose first gather succeeded, whose
+// second did, and the hexes added by all threads in the first.
+__global__ void __launch_bounds__(NODE_THREADS) k_selftest_gather(Mesh m, const double* groups, int stages, int late,
+                                                                  unsigned long long limit, int* out) {
+    __shared__ GatherSmem S;
+    gather_init(S);
+    if (threadIdx.x == 0 && late >= 0 && late < 4)
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], 16;" ::"r"(smem_addr(&S.full[late])) : "memory");
+    int i = 0, j = 0, k = 0;
+    const bool active = threadIdx.x < m.nn;
+    if (active) split3(threadIdx.x, m.nnx, m.nny, i, j, k);
+    for (int pass = 0; pass < 2; pass++) {
+        const Gather<HEAT_CHUNK, HEAT_TAIL> G{S, groups, HROWS, stages,
+                                              gather_groups(NODE_THREADS) * (HEAT_CHUNK + HEAT_TAIL) * GROUP,
+                                              (unsigned)pass, limit};
+        int added = 0;
+        const bool ok = G.run(m, 0, active, i, j, k, [&](int, const double* r) { added += *r == 0.0; });
+        if (ok) atomicAdd(out + pass, 1);
+        if (pass == 0 && added) atomicAdd(out + 2, added);
+        __syncthreads();
+        if (S.gave_up) break;
+    }
+}
+
 // ---- host transfers: node fields between the packed double4 layout and
 // the reference's interleaved (x, y, z) / scalar arrays -------------------------------------
 // what: 0 = x, y, z of each double4 <-> 3 doubles per node; 1 = w <-> 1 double per node
