@@ -1715,14 +1715,24 @@ int snac_gpu_step_host(snac_gpu* h, const snac_state_view* in, const snac_state_
     const size_t vbytes = h->abi >= 2 ? sizeof(snac_state_view) : offsetof(snac_state_view, plastic_strain_tensor);
     memcpy(&vi, in, vbytes);
     memcpy(&vo, out, vbytes);
-    // default: one slab per 6 MiB of stresses (the bulk of the transfers),
-    // up to 16 slabs; smaller slabs cost more in per-slab latency than they
-    // save in pipeline fill, but below six slabs the fill weighs more: one per 3 MiB there
-    // (45x21x37 visco-plastic: 3 slabs 1.03 ms, 6 slabs 0.95, 8 slabs 0.98)
+    // default: one slab per 6 MiB of stresses (the bulk of the transfers), up to
+    // 16 slabs; smaller slabs cost more in per-slab latency than they save in
+    // pipeline fill.  Below six slabs the fill weighs more: one per 3 MiB
+    // there.  Below 8 MiB the latencies of a second slab cost what the overlap gives.
+    // ms by slabs, the rule's in brackets:
+    //   MiB                      1       2      3       4       5       6      8
+    //   4.6 visco-plastic      [0.382]  0.399  0.413   0.412   0.446   0.459  0.496
+    //   6.6 plastic            [0.445]  0.448  0.442   0.425   0.435   0.450  0.456
+    //   6.6 visco-plastic      [0.494]  0.514  0.512   0.506   0.522
+    //   9.5 visco-plastic       0.655   0.675 [0.661]  0.643   0.652
+    //   13.2 plastic            0.824   0.813  0.777  [0.758]  0.763
+    //   16.0 visco-plastic      1.024   1.043  1.022   0.970  [0.940]  0.950  0.932
+    //   34.7 plastic            2.056   2.016  1.844   1.796   1.713  [1.696] 1.690
     const long long stress_bytes = h->mesh.ne * NT * 6 * (long long)sizeof(double);
     auto slabs_of = [&](long long unit) { return (stress_bytes + unit / 2) / unit; };
-    const int S = chunks ? chunks
-                         : (int)std::max({1LL, std::min(6LL, slabs_of(3LL << 20)), std::min(16LL, slabs_of(6LL << 20))});
+    const int S = chunks                         ? chunks
+                  : stress_bytes < (8LL << 20)   ? 1
+                                                 : (int)std::max(std::min(6LL, slabs_of(3LL << 20)), std::min(16LL, slabs_of(6LL << 20)));
     {
         // every return below waits for this call's copies first: the caller
         // may release its host buffers once the call has returned
