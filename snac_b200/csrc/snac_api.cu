@@ -302,12 +302,13 @@ unsigned node_blocks(const Mesh& m) { return (unsigned)((m.nn + NODE_THREADS - 1
 constexpr int force_rows(int dt_type, bool vonly) {
     return force_chunk(dt_type == SNAC_DT_CONSTANT) + force_tail(dt_type == SNAC_DT_CONSTANT, vonly);
 }
-// The minimum length scale takes a thread per tet while its blocks (12 hexes)
-// fit one wave of the GPU (8 resident per SM), a thread per hex beyond.
-#ifndef MINLS_TET
-#define MINLS_TET 8
-#endif
-constexpr int MINLS_TET_BLOCKS_PER_SM = MINLS_TET;
+// The minimum length scale takes a thread per tet up to this many blocks (of 12 hexes)
+// per SM, a thread per hex beyond.  us a step of an elastic model, per tet /
+// per hex: 512 hexes 13.7 / 16.3, 4096 16.9 / 18.9, 10,648 22.9 / 24.0, 13,824 24.5 /
+// 25.2; the forms meet between 16,224 (27.0 / 27.2) and 20,384 (31.2 / 31.2);
+// 28,672 38.8 / 37.4, 131,072 145 / 134.  (66 registers let seven blocks be resident.)
+constexpr int MINLS_TET_BLOCKS_PER_SM = 8;
+
 // of a node gather: its most stages
 constexpr size_t most_stages(int rows) { return GATHER_STAGES * gather_stage_bytes(rows, NODE_THREADS); }
 static_assert(most_stages(CCHUNK) <= 227 * 1024, "the widest gather's stages fit an SM");

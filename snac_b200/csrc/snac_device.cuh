@@ -133,10 +133,6 @@ __device__ __forceinline__ void report(DevScalars* sc, int code, long long index
     }
 }
 
-#ifndef SNAC_MARKSTEIN_DIV
-#define SNAC_MARKSTEIN_DIV 2
-#endif
-
 // ---- correctly rounded division by a known reciprocal --------------------------------
 // With z = RN(1/y) (the correctly rounded reciprocal) and q0 = RN(x z),
 // which is within one ulp of x / y, the remainder r = x - q0 y is exact in
@@ -150,8 +146,7 @@ __device__ __forceinline__ void report(DevScalars* sc, int code, long long index
 // range without overflow or underflow: operands outside a safe exponent
 // window and negative divisors (checked with integer operations on the high
 // and low words) take the IEEE division; zeros get their sign from the form
-// of the correction step (markstein() below).  SNAC_MARKSTEIN_DIV = 1
-// uses it for the constant divisors only, 2 also for shared divisors.  The device self-test
+// of the correction step (markstein() below).  The device self-test
 // (snac_gpu_selftest_division) compares every helper with the hardware '/'
 // on random operands, near-ties included.
 
@@ -221,28 +216,18 @@ __host__ __device__ __forceinline__ double markstein(double x, double y, double 
 
 // RN(x / c) for a constant c with z = RN(1/c) and 1 <= c <= 16
 __host__ __device__ __forceinline__ double dvk(double x, double c, double z) {
-#if SNAC_MARKSTEIN_DIV >= 1
     const double q0 = x * z;
     const double q = markstein(x, c, z, q0);
     if (!zero_or_within<-900, 900>(x)) return ieee_div(x, c);
     return q;
-#else
-    (void)z;
-    return x / c;
-#endif
 }
 
 // RN(x / y) given z = RN(1/y)
 __host__ __device__ __forceinline__ double dvz(double x, double y, double z) {
-#if SNAC_MARKSTEIN_DIV >= 2
     const double q0 = x * z;
     const double q = markstein(x, y, z, q0);
     if (!(zero_or_within<-450, 450>(x) && positive_within<-450, 450>(y))) return ieee_div(x, y);
     return q;
-#else
-    (void)z;
-    return x / y;
-#endif
 }
 
 // The same window as one unsigned compare of a key, x != 0 only, so that a
@@ -275,7 +260,7 @@ __device__ __forceinline__ bool all_zero_or_within(const double (&x)[N]) {
 // the IEEE division for all of its members.
 template <int N>
 __host__ __device__ __forceinline__ void dvk_n(double (&x)[N], double c, double z) {
-#if defined(__CUDA_ARCH__) && SNAC_MARKSTEIN_DIV >= 1
+#ifdef __CUDA_ARCH__
     double q[N];
 #pragma unroll
     for (int i = 0; i < N; i++) q[i] = markstein(x[i], c, z, x[i] * z);
@@ -293,7 +278,7 @@ __host__ __device__ __forceinline__ void dvk_n(double (&x)[N], double c, double 
 }
 template <int N>
 __host__ __device__ __forceinline__ void dvz_n(double (&x)[N], double y, double z) {
-#if defined(__CUDA_ARCH__) && SNAC_MARKSTEIN_DIV >= 2
+#ifdef __CUDA_ARCH__
     double q[N];
 #pragma unroll
     for (int i = 0; i < N; i++) q[i] = markstein(x[i], y, z, x[i] * z);
@@ -352,14 +337,6 @@ struct TetGeom {
     double A[4];
     V3 n[4];
 };
-
-__device__ __forceinline__ void tet_geometry(const V3 c[4], TetGeom& g) {
-    g.V = tet_volume(c[0], c[1], c[2], c[3]);
-    g.zV = recip(g.V);
-#pragma unroll
-    for (int f = 0; f < 4; f++)
-        tet_face(c[face_node(f, 0)], c[face_node(f, 1)], c[face_node(f, 2)], g.A[f], g.n[f]);
-}
 
 // ---- the same geometry for tame coordinates ------------------------------------------
 // A coordinate is tame when it is 0 or its magnitude lies in [2^-100, 2^100)

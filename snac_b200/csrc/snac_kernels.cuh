@@ -129,10 +129,7 @@ struct Config {
 __host__ __device__ constexpr int elem_minb(int plugin) {
     return plugin == SNAC_RHEOLOGY_ELASTIC || plugin == SNAC_RHEOLOGY_MAXWELL ? 5 : 4;
 }
-#ifndef SNAC_ELEM_WARPS
-#define SNAC_ELEM_WARPS 4
-#endif
-constexpr int ELEM_WARPS = SNAC_ELEM_WARPS;    // warps per block in the element kernels
+constexpr int ELEM_WARPS = 4;                   // warps per block in the element kernels
 constexpr int ELEM_PER_BLOCK = ELEM_WARPS * 3;  // 12 elements per block
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int FROWS_MAX = 170;
@@ -1217,8 +1214,6 @@ inline __device__ __noinline__ V3 traction_force(const double4* pos, int nx, int
     return V3{fx, fy, fz};
 }
 
-// VONLY: cfg.vonly (a template argument, so that the gather loop of each
-// instance is straight-line code)
 // The tail of the node loop for node n with its summed force and inertial
 // mass: force-BC plugins, FLAC local damping with the pre-update velocity
 // (UpdateNode.c:102-104), v and x update, BC override; returns the node's
