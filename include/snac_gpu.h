@@ -367,6 +367,11 @@ int  snac_gpu_fp64_rate(double* fma_per_second);
  * signed zeros, exact quotients and ties) compared bit for bit with the
  * IEEE quotient of the GPU; *mismatches receives the count (expected 0). */
 int  snac_gpu_selftest_division(long long n, unsigned long long seed, long long* mismatches);
+/* The short square root and reciprocals of the element kernels at n (up to
+ * 2^24) given operands: root[i] and recip_root[i] the root of q[i] and its
+ * reciprocal (q in [2^-714, 2^408]), recip[i] the reciprocal of q[i] itself (q in [1,
+ * 2^64]); operands outside these ranges give meaningless values. */
+int  snac_gpu_selftest_roots(const double* q, long long n, double* root, double* recip_root, double* recip);
 /* Self-test of the bounded wait of the node gathers (csrc/snac_kernels.cuh):
  * one block gathers a mesh of 3x2x3 hexes twice, with 1, 2 or 4 stages.  The
  * pair of hexes `late` (0 to 3; another value: none) never completes, so its wait runs

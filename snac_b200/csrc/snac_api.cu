@@ -896,6 +896,22 @@ double hydrostatic_ic(const snac_gpu_desc* d, const std::vector<double>& coord, 
 
 extern "C" {
 
+int snac_gpu_selftest_roots(const double* q, long long n, double* root, double* recip_root, double* recip) {
+    if (!q || !root || !recip_root || !recip || n < 1 || n > (1LL << 24)) return SNAC_GPU_EINVAL;
+    const size_t bytes = (size_t)n * sizeof(double);
+    double* d = nullptr;  // [4][n]
+    if (cudaMalloc(&d, 4 * bytes) != cudaSuccess) return SNAC_GPU_ENOMEM;
+    cudaError_t e = cudaMemcpy(d, q, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_selftest_roots<<<(unsigned)((n + 127) / 128), 128>>>(n, d, d + n, d + 2 * n, d + 3 * n);
+        e = cudaGetLastError();
+    }
+    double* const out[3] = {root, recip_root, recip};
+    for (int a = 0; a < 3 && e == cudaSuccess; a++) e = cudaMemcpy(out[a], d + (a + 1) * n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : SNAC_GPU_ECUDA;
+}
+
 int snac_gpu_selftest_gather(int stages, int late, double limit_ms, int* status, int counts[3]) {
     if (!status || !counts || (stages != 1 && stages != 2 && stages != 4) || !(limit_ms >= 0.0 && limit_ms <= 1000.0))
         return SNAC_GPU_EINVAL;

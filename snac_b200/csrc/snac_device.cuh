@@ -367,11 +367,19 @@ __device__ __forceinline__ bool tame_size(double x) {
 // s = RN(sqrt(q)) and z = RN(1/s) for q in [2^-714, 2^408]: Newton's coupled
 // iteration for sqrt(q) and 1/(2 sqrt(q)) from the hardware's approximate
 // reciprocal root (its error e goes to about 3/2 e^2 per pass: two passes
-// from 2^-20 reach rounding level), then Markstein's final steps, one FMA
-// each: s = RN(g + (q - g^2) h), and y + y (1 - s y) for the reciprocal,
-// which is RN(1/s) unless s has an all-ones significand (P. Markstein, IBM
-// J. Res. Dev. 34(1), 1990).  The device self-test compares both with the
-// IEEE root and quotient.
+// from 2^-20 reach rounding level), then a final step each in the manner of
+// Markstein (IBM J. Res. Dev. 34(1), 1990): s = RN(g + (q - g^2) h), and
+// z = RN(y + y (e + e^2)) with e = 1 - s y.
+//
+// y may be 3.5 2^-53 (relative) from 1/s: 2^-53 for each of four roundings, half of them
+// halved (g and h of the first pass and q y; h of the second; s).  y + y e is 1/s
+// (1 - e^2): without the e^2 it is off by up to 12 2^-106, which is too much for some
+// significands b whose product with a midpoint m (54 bits) comes that near to a power of
+// two.  With it the error is what rounding e and e + e^2 leaves, under 5
+// 2^-106: each b that has such an m within 24 (they follow from the factors of
+// 2^k + j) then gives RN(1/s) for every y in that range, but for the all-ones significand.
+// The self-test of the roots takes those b, and the q nearest to the square of
+// a midpoint, on the device (snac_gpu_selftest_roots).
 __device__ __forceinline__ void sqrt_recip(double q, double& s, double& z) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
@@ -384,11 +392,13 @@ __device__ __forceinline__ void sqrt_recip(double q, double& s, double& z) {
     h = fma(h, r, h);
     s = fma(fma(-g, g, q), h, g);
     y = h + h;
-    z = fma(fma(-s, y, 1.0), y, y);
+    const double e = fma(-s, y, 1.0);
+    z = fma(fma(e, e, e), y, y);
 }
 
 // z = RN(1/y) for y in [1, 2^64] whose low word is not all ones: Newton from
-// the hardware's approximate reciprocal, the last step Markstein's (see sqrt_recip).
+// the hardware's approximate reciprocal, the last step Markstein's.  (Two steps
+// leave r within one rounding of 1/y, where y + y e needs no further term.)
 __device__ __forceinline__ double recip_mid(double y) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));

@@ -225,6 +225,14 @@ __global__ void k_selftest_division(long long n, unsigned long long seed, unsign
     if (local) atomicAdd(bad, local);
 }
 
+// the short root and reciprocals of n given operands
+__global__ void k_selftest_roots(long long n, const double* q, double* root, double* recip_root, double* recip) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    sqrt_recip(q[i], root[i], recip_root[i]);
+    recip[i] = recip_mid(q[i]);
+}
+
 // ---- self-test of the gather's bounded wait ---------------------------------------------
 // One block gathers a small mesh's heat groups twice, with `stages` stages and
 // `limit` ns for each wait.  The barrier of pair `late` (none if it is not 0 to 3) is
