@@ -42,10 +42,16 @@ def snac_tree() -> str:
     return os.path.normpath(os.path.join(HERE, "..", "..", "reference", "Snac"))
 
 
+class CheckerMissing(RuntimeError):
+    """A checker that compiles from the SNAC tree, on a machine without it."""
+
+
 def build(kind: str = "port") -> str:
     """Compile the checker with oracle/Makefile if it is missing."""
     path = PATHS[kind]
     if not os.path.exists(path):
+        if kind != "port" and not os.path.isdir(snac_tree()):
+            raise CheckerMissing(f"the {kind} checker is not built and there is no SNAC tree at {snac_tree()}")
         target = {"port": "all", "plugin_host": "plugin"}.get(kind, "ref")
         subprocess.run(["make", "-s", "-C", HERE, target, f"SNAC_REF={snac_tree()}"], check=True)
     return path
