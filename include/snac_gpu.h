@@ -400,9 +400,9 @@ int  snac_gpu_selftest_gather(int stages, int late, double limit_ms, int* status
  * scale enters them; snac_gpu_adjoint_grads also returns the gradients with
  * respect to the initial state.)
  * Device memory: a call (snac_gpu_misfit too) allocates one workspace, for
- * the states it keeps and the adjoints.  It stays with the handle for the
- * next call while all handles of the process keep 512 MiB at most, else it is
- * released when the call ends; snac_gpu_destroy releases it. */
+ * the states it keeps and the adjoints.  One of up to 512 MiB stays with the
+ * handle for the next call while all handles of the process keep 2 GiB at
+ * most; any other is released when the call ends.  snac_gpu_destroy releases it. */
 typedef struct snac_adjoint_desc {
     int nsteps;
     int checkpoint_every;

@@ -2396,11 +2396,12 @@ struct Carver {
         used += ((size_t)n * sizeof(T) + 255) & ~(size_t)255;
     }
 };
-// A call's workspace stays with its handle for the next call while the handles of the process
-// keep this much in all; one that would exceed it is released when its call
-// ends.  32x16x32, 60 steps: 12.4 ms a call with it kept, 13.5 without;
-// 10x6x8, 24 steps: 2.5 and 3.2; a misfit 0.03 and 0.7.
-constexpr size_t ADJ_KEEP = (size_t)512 << 20;
+// A call's workspace of up to ADJ_KEEP stays with its handle for the next call while the
+// handles of the process keep ADJ_KEEP_ALL in all; any other is released when
+// its call ends.  32x16x32, 60 steps (240 MB): 12.4 ms a call with it kept, 13.5 without;
+// 10x6x8, 24 steps: 2.5 and 3.2; 48x24x40, 60 steps (660 MB): 30.3 and 30.6; a misfit 0.03
+// and 0.7.  (Several handles of 240 MB used in turn, with room for two of them: 15.1 ms a call.)
+constexpr size_t ADJ_KEEP = (size_t)512 << 20, ADJ_KEEP_ALL = (size_t)2 << 30;
 std::atomic<size_t> g_adj_kept{0};
 
 void adj_ws_release(snac_gpu* h) {
@@ -2426,7 +2427,7 @@ int adj_ws_reserve(snac_gpu* h, size_t bytes) {
 void adj_ws_trim(snac_gpu* h) {
     if (!h->adj_ws || h->adj_ws_kept) return;
     size_t kept = g_adj_kept.load();
-    while (kept + h->adj_ws_bytes <= ADJ_KEEP)
+    while (h->adj_ws_bytes <= ADJ_KEEP && kept + h->adj_ws_bytes <= ADJ_KEEP_ALL)
         if (g_adj_kept.compare_exchange_weak(kept, kept + h->adj_ws_bytes)) {
             h->adj_ws_kept = true;
             return;
