@@ -53,20 +53,20 @@ NODES_PER_HEX = {"c1": 2601 / 2048, "c2": 139425 / 131072, "c3": 1081665 / 10485
 # DRAM bytes (read + write) of one launch of the dominant kernel, from one
 # ncu capture of that kernel on the same workload
 # (profiles/k_fused_step_plastic_64x32x64.md); None where none was taken.
-NCU_TRAFFIC = {("c2", "k_fused_step"): 83.453440e6 + 149.549824e6,
-               ("c3", "k_fused_stress"): 656.603392e6 + 1701.246208e6}
+NCU_TRAFFIC = {("c2", "k_fused_step"): 83.447552e6 + 150.336256e6,
+               ("c3", "k_fused_stress"): 656.682496e6 + 1704.077312e6}
 # what bounds the dominant kernel instead of HBM, from the same kind of ncu
 # capture (fractions of peak; profiles/k_fused_step_plastic_64x32x64.md,
 # profiles/k_fused_stress_viscoplastic_128x64x128.md)
-NCU_PIPES = {("c2", "k_fused_step"): {"fp64_pipe": 0.485, "issue_active": 0.572, "dram_throughput": 0.243},
-             ("c3", "k_fused_stress"): {"fp64_pipe": 0.509, "issue_active": 0.605, "dram_throughput": 0.283}}
+NCU_PIPES = {("c2", "k_fused_step"): {"fp64_pipe": 0.501, "issue_active": 0.567, "dram_throughput": 0.251},
+             ("c3", "k_fused_stress"): {"fp64_pipe": 0.524, "issue_active": 0.594, "dram_throughput": 0.291}}
 # FP64 instructions (thread level: DADD, DMUL, DFMA) of one launch of the
 # dominant kernel, from one ncu capture of it on the same workload
 # (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum); None
 # where none was taken.  With the device's FP64 rate, measured live by
 # snac_gpu_fp64_rate, they give the kernel's FP64 roofline.
-NCU_FP64 = {("c2", "k_fused_step"): {"dadd": 367450200, "dmul": 376451230, "dfma": 196439232},
-            ("c3", "k_fused_stress"): {"dadd": 3364227624, "dmul": 3435901488, "dfma": 2309681024}}
+NCU_FP64 = {("c2", "k_fused_step"): {"dadd": 364566049, "dmul": 373479216, "dfma": 202031808},
+            ("c3", "k_fused_stress"): {"dadd": 3341487680, "dmul": 3401606496, "dfma": 2354420608}}
 ARITHMETIC = {
     "c1": "reference rounding (no FMA contraction), bitwise equal to the CPU oracle",
     "c2": "reference rounding (no FMA contraction), bitwise equal to the CPU oracle",

@@ -121,9 +121,9 @@ struct Config {
 };
 
 // Resident blocks per SM asked of the compiler (the register budget).  Elastic
-// and Maxwell at 5 (96 registers, 60 bytes of spills): 84 against 88 us at
-// 131 k hexes elastic; the hooks with a return map at 4 (128 registers, no
-// spills to speak of): 104 against 109 us plastic, 128 against 141 us
+// and Maxwell at 5 (96 registers, 56 and 24 bytes of spills): 84 against 88 us at
+// 131 k hexes elastic; the hooks with a return map at 4 (128 registers, 8 bytes
+// of spills plastic, 40 visco-plastic): 104 against 109 us plastic, 128 against 141 us
 // visco-plastic, whose spills at 96 registers miss the small L1 that the
 // shared memory leaves.
 __host__ __device__ constexpr int elem_minb(int plugin) {
